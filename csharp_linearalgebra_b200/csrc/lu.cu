@@ -27,6 +27,7 @@
 #include "batch.cuh"
 #include "device_util.cuh"
 #include "lu_panel.h"
+#include "subst_cols.h"
 #include "tns_internal.h"
 
 #include <algorithm>
@@ -592,8 +593,8 @@ __global__ void trsm_kernel(const __grid_constant__ Batch<TrsmDesc> bt) {
 // order of k, and the chains of different (row, column) pairs are
 // independent. The rows are cut into blocks of 32; for each block, in the
 // order of k:
-//   1. subst_diag_kernel solves the block's own triangle, which completes
-//      x[k] for every k of the block;
+//   1. solve_diag_blocks (subst_cols.cu) solves the block's own triangle,
+//      which completes x[k] for every k of the block;
 //   2. subst_update_kernel applies the block's steps to every row beyond it,
 //      continuing each row's chain from the value it holds, steps in order.
 // Blocking regroups whole chains and never reorders one, so every x[i] sees
@@ -602,15 +603,7 @@ __global__ void trsm_kernel(const __grid_constant__ Batch<TrsmDesc> bt) {
 // register-tiled product on every SM. The adjoint solves accumulate row by
 // row in the reference (dot products), an order a right-looking sweep cannot
 // reproduce; they stay on the blocked GEMM path.
-constexpr int kSubstBlock = 32;
-
-struct SubstDiagDesc {
-    const double* f;  // the factors (ld ldf)
-    int ldf;
-    double* x;  // right-hand sides (ld ldx), overwritten
-    int ldx, nrhs;
-    int k0, w;  // the block: rows and steps [k0, k0 + w)
-};
+constexpr int kSubstBlock = kDiagBlock;
 
 struct SubstUpdateDesc {
     const double* f;
@@ -628,78 +621,6 @@ template <bool CPLX>
 __device__ __forceinline__ Z subst_axpy(Z x, Z nxk, Z f) {
     if (!CPLX) return Z{add_rn(x.re, mul_rn(nxk.re, f.re)), 0.0};
     return zadd(x, zmul(nxk, f));
-}
-
-// Step 1: the block's own triangle, one thread per right-hand side column,
-// the block's values in registers and its triangle in shared memory (every
-// thread reads the same entry at a time: a broadcast).
-template <bool CPLX, bool UPPER, bool LDIV = false>
-__global__ void __launch_bounds__(128) subst_diag_kernel(const __grid_constant__ Batch<SubstDiagDesc> b) {
-    constexpr int B = kSubstBlock;
-    constexpr int ES = CPLX ? 2 : 1;
-    const SubstDiagDesc& d = batch_item(b, blockIdx.y);
-    if ((int)(blockIdx.x * blockDim.x) >= d.nrhs) return;  // whole block idle
-    const int w = d.w;
-    __shared__ Z t[B][B];  // t[k][i] = F[k0 + i, k0 + k]
-    for (int e = threadIdx.x; e < B * B; e += blockDim.x) {
-        const int k = e / B, i = e % B;
-        Z v{0.0, 0.0};
-        if (i < w && k < w) {
-            const double* p = d.f + ((size_t)(d.k0 + k) * d.ldf + d.k0 + i) * ES;
-            v = Z{p[0], CPLX ? p[1] : 0.0};
-        }
-        t[k][i] = v;
-    }
-    __syncthreads();
-    const int col = blockIdx.x * blockDim.x + threadIdx.x;
-    if (col >= d.nrhs) return;
-    double* x = d.x + ((size_t)col * d.ldx + d.k0) * ES;
-    Z v[B];
-#pragma unroll
-    for (int i = 0; i < B; ++i) {
-        v[i] = Z{0.0, 0.0};
-        if (i < w) v[i] = Z{x[(size_t)i * ES], CPLX ? x[(size_t)i * ES + 1] : 0.0};
-    }
-    if (!UPPER) {
-#pragma unroll
-        for (int k = 0; k < B; ++k) {
-            if (k >= w) continue;
-            if (LDIV) {
-                // An explicit diagonal (Triangular.SolveLower, Triangular.cs:131-150;
-                // the adjoint's U^H): x_k /= f_kk first, always for real, and for
-                // complex when x_k is not zero (BlockedLu's division rule).
-                const Z dg = t[k][k];
-                if (!CPLX) v[k].re = __ddiv_rn(v[k].re, dg.re);
-                else if (!(v[k].re == 0.0 && v[k].im == 0.0)) v[k] = zdiv(v[k], dg);
-            }
-            const Z xk = v[k];
-            if (k == B - 1 || (xk.re == 0.0 && xk.im == 0.0)) continue;
-            const Z nxk{-xk.re, -xk.im};
-#pragma unroll
-            for (int i = k + 1; i < B; ++i)
-                if (i < w) v[i] = subst_axpy<CPLX>(v[i], nxk, t[k][i]);
-        }
-    } else {
-#pragma unroll
-        for (int k = B - 1; k >= 0; --k) {
-            if (k >= w) continue;
-            Z xk = v[k];
-            const Z dg = t[k][k];
-            if (!CPLX) xk.re = __ddiv_rn(xk.re, dg.re);
-            else if (!(xk.re == 0.0 && xk.im == 0.0)) xk = zdiv(xk, dg);
-            v[k] = xk;
-            if (xk.re == 0.0 && xk.im == 0.0) continue;
-            const Z nxk{-xk.re, -xk.im};
-#pragma unroll
-            for (int i = 0; i < k; ++i) v[i] = subst_axpy<CPLX>(v[i], nxk, t[k][i]);
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < B; ++i)
-        if (i < w) {
-            x[(size_t)i * ES] = v[i].re;
-            if (CPLX) x[(size_t)i * ES + 1] = v[i].im;
-        }
 }
 
 // Asynchronous 16- or 8-byte copies global -> shared; src_bytes 0 fills the
@@ -1045,16 +966,8 @@ void launch_trsm(Context& ctx, bool cplx, int kind, std::vector<TrsmDesc>& v) {
 
 // One block step of the substitution for every item of a batch: the
 // diagonal blocks in one launch, then the updates of all items' tiles in one.
-template <bool CPLX, bool UPPER, bool LDIV = false>
-void launch_subst_step_t(Context& ctx, std::vector<SubstDiagDesc>& diag, std::vector<SubstUpdateDesc>& upd) {
-    if (!diag.empty()) {
-        int mr = 0;
-        for (auto& d : diag) mr = std::max(mr, d.nrhs);
-        Batch<SubstDiagDesc> b = make_batch(ctx, diag);
-        subst_diag_kernel<CPLX, UPPER, LDIV><<<dim3((mr + 127) / 128, b.count), 128, 0, ctx.stream>>>(b);
-        TNS_CUDA(cudaGetLastError());
-        ctx.kernel_launches++;
-    }
+template <bool CPLX, bool UPPER>
+void launch_subst_update_t(Context& ctx, std::vector<SubstUpdateDesc>& upd) {
     if (!upd.empty()) {
         long long total = 0;
         for (auto& u : upd) {
@@ -1078,15 +991,10 @@ void launch_subst_step_t(Context& ctx, std::vector<SubstDiagDesc>& diag, std::ve
 
 void launch_subst_step(Context& ctx, bool cplx, bool upper, std::vector<SubstDiagDesc>& diag,
                        std::vector<SubstUpdateDesc>& upd, bool lower_divides = false) {
-    if (cplx) {
-        if (upper) launch_subst_step_t<true, true>(ctx, diag, upd);
-        else if (lower_divides) launch_subst_step_t<true, false, true>(ctx, diag, upd);
-        else launch_subst_step_t<true, false>(ctx, diag, upd);
-    } else {
-        if (upper) launch_subst_step_t<false, true>(ctx, diag, upd);
-        else if (lower_divides) launch_subst_step_t<false, false, true>(ctx, diag, upd);
-        else launch_subst_step_t<false, false>(ctx, diag, upd);
-    }
+    solve_diag_blocks(ctx, cplx, upper ? LowerKind::kNone : lower_divides ? LowerKind::kDivide : LowerKind::kUnit, upper,
+                      diag);
+    if (cplx) upper ? launch_subst_update_t<true, true>(ctx, upd) : launch_subst_update_t<true, false>(ctx, upd);
+    else upper ? launch_subst_update_t<false, true>(ctx, upd) : launch_subst_update_t<false, false>(ctx, upd);
 }
 
 // One block step's panels. Up to row_panel_max_rows() rows they are factored
@@ -1139,162 +1047,72 @@ struct SubstItem {
     double* x;
     int ldx, n, nrhs;
 };
-// The whole complex substitution in one launch for a few right-hand sides:
-// one warp per pair of them (a half-warp each), the pair's columns in shared
-// memory, and the factor column each step reads (diagonal included) copied in
-// by cp.async kStageAhead steps ahead into a ring of kStageSlots. Step p
-// finishes x[p] (the division first where the blocked kernels divide) and,
-// unless x[p] is zero, applies subst_axpy(x[i], -x[p], f[i, p]) to every
-// later row (lower: rows below, upper: rows above) -- each row's chain in the
-// blocked kernels' order, so the same bits, with no launch per 32-row block.
-// Real right-hand sides stay on the blocked kernels, which measured as fast
-// (n = 512, 8 right-hand sides: 1.1 ms per solve call against 1.25 ms).
-// The staged kernels (this one and the left-looking ones below) copy the
-// factor column of step s + kStageAhead while step s runs, into a ring of
-// kStageSlots columns: far enough ahead that the copies' latency is hidden.
+// The staged left-looking kernels below copy the factor column of step s +
+// kStageAhead while step s runs, into a ring of kStageSlots columns: far
+// enough ahead that the copies' latency is hidden.
 constexpr int kStageSlots = 6;
 constexpr int kStageAhead = kStageSlots - 1;
-constexpr int kSubstFusedMaxN = 1536;  // complex: 6 slots + 2 columns = 192 KB
-constexpr int kSubstFusedMaxRhs = 16;
 
-struct SubstFusedDesc {
-    const double* f;
-    int ldf;
-    double* x;
-    int ldx, n, nrhs;
-};
+// A batch with many more columns than the GPU takes at once in the one-launch
+// solve (ctas: its CTAs of eight columns, each keeping a whole SM): there the
+// columns alone fill the GPU, and what counts is FP64 work per column. So the
+// triangles run one thread per column, and the updates, nearly all of the
+// work, on the tiled kernel, which shares each factor entry between 64
+// columns: 32-row blocks within blocks of kWideBlock rows, then the rows beyond
+// take kWideBlock steps in one launch (per 64 sweep matrices 12.5 ms of
+// updates at 128 steps a launch against 16.1 ms at 32; the one-launch solve
+// took 22 ms of the whole GPU).
+constexpr int kWideBlock = 128;
+bool wide_batch(Context& ctx, const std::vector<SubstItem>& items) {
+    long long ctas = 0;
+    for (auto& it : items)
+        if (it.n > 2 * kWideBlock) ctas += (it.nrhs + 7) / 8;
+    return ctas >= 2 * ctx.num_sms;
+}
 
-template <bool CPLX, bool UPPER, bool LDIV>
-__global__ void __launch_bounds__(32) subst_fused_kernel(const __grid_constant__ Batch<SubstFusedDesc> b, int nmax) {
-    using E = typename std::conditional<CPLX, double2, double>::type;
-    const SubstFusedDesc& d = batch_item(b, blockIdx.y);
-    const int n = d.n;
-    if ((int)blockIdx.x * 2 >= d.nrhs || n == 0) return;  // the whole warp
-    extern __shared__ __align__(16) double ssm[];
-    E* slots = reinterpret_cast<E*>(ssm);  // kStageSlots x nmax (nmax: the batch's largest order)
-    E* xs = slots + kStageSlots * nmax;    // 2 x nmax
-    const int lane = threadIdx.x, L = lane & 15, h = lane >> 4;
-    const int col = blockIdx.x * 2 + h;
-    const bool active = col < d.nrhs;
-    // A half past the last column works on a copy of the pair's first column
-    // and never writes it back.
-    E* xg = reinterpret_cast<E*>(d.x) + (size_t)(active ? col : blockIdx.x * 2) * d.ldx;
-    E* y = xs + h * nmax;
-    for (int p = L; p < n; p += 16) y[p] = xg[p];
-    // Step s reads column p of the factor over rows [p, n) (lower) or [0, p]
-    // (upper), the diagonal at p either way.
-    auto issue = [&](int s) {
-        if (s < n) {
-            const int p = UPPER ? n - 1 - s : s;
-            const int r0 = UPPER ? 0 : p, cnt = UPPER ? p + 1 : n - p;
-            const E* src = reinterpret_cast<const E*>(d.f) + (size_t)p * d.ldf + r0;
-            E* dst = slots + (size_t)(s % kStageSlots) * nmax;
-            for (int q = lane; q < cnt; q += 32) {
-                if constexpr (CPLX) cp_async16(dst + q, src + q, true);
-                else cp_async8(dst + q, src + q, true);
-            }
-        }
-        cp_async_commit();
+void substitute_wide(Context& ctx, bool cplx, bool upper, bool lower_divides, const std::vector<SubstItem>& items) {
+    constexpr int B = kWideBlock, D = kSubstBlock;
+    int steps = 0;
+    for (auto& it : items) steps = std::max(steps, (it.n + B - 1) / B);
+    // Rows [r0, r1) of an item take the steps [k0, k1).
+    auto update = [](const SubstItem& it, int r0, int r1, int k0, int k1) {
+        return SubstUpdateDesc{it.f, it.ldf, it.x, it.ldx, it.nrhs, r0, r1, k0, k1, (r1 - r0 + 63) / 64, 0};
     };
-    for (int q = 0; q < kStageAhead; ++q) issue(q);
-    for (int s = 0; s < n; ++s) {
-        issue(s + kStageAhead);
-        cp_async_wait<kStageAhead>();
-        __syncwarp();
-        const int p = UPPER ? n - 1 - s : s;
-        const int r0 = UPPER ? 0 : p;
-        const E* fc = slots + (size_t)(s % kStageSlots) * nmax;  // fc[r - r0] = f[r, p]
-        Z xk;
-        {
-            const E v = y[p];
-            if constexpr (CPLX) xk = Z{v.x, v.y};
-            else xk = Z{v, 0.0};
-        }
-        if (UPPER || LDIV) {
-            // x_p /= f_pp: always for real; for complex when x_p is not zero.
-            const E dv = fc[p - r0];
-            if constexpr (!CPLX) {
-                xk.re = __ddiv_rn(xk.re, dv);
-            } else {
-                if (!(xk.re == 0.0 && xk.im == 0.0)) xk = zdiv(xk, Z{dv.x, dv.y});
-            }
-        }
-        if (!(xk.re == 0.0 && xk.im == 0.0)) {
-            const Z nxk{-xk.re, -xk.im};
-            const int i0 = UPPER ? 0 : p + 1, i1 = UPPER ? p : n;
-            auto update = [&](int i, E fv, E xv) {
-                if constexpr (CPLX) {
-                    const Z r = subst_axpy<true>(Z{xv.x, xv.y}, nxk, Z{fv.x, fv.y});
-                    y[i] = make_double2(r.re, r.im);
-                } else {
-                    y[i] = subst_axpy<false>(Z{xv, 0.0}, nxk, Z{fv, 0.0}).re;
+    for (int s = 0; s < steps; ++s)
+        for (int d = 0; d < B / D; ++d) {
+            std::vector<SubstDiagDesc> diag;
+            std::vector<SubstUpdateDesc> upd;
+            for (auto& it : items) {
+                const int n = it.n, blocks = (n + B - 1) / B;
+                if (n == 0 || it.nrhs == 0 || s >= blocks) continue;
+                const int b0 = (upper ? blocks - 1 - s : s) * B, b1 = std::min(n, b0 + B);
+                const int inner = (b1 - b0 + D - 1) / D;
+                if (d >= inner) continue;
+                const int k0 = b0 + (upper ? inner - 1 - d : d) * D, k1 = std::min(b1, k0 + D);
+                diag.push_back(SubstDiagDesc{it.f, it.ldf, it.x, it.ldx, it.nrhs, k0, k1 - k0});
+                if (d + 1 < inner) {
+                    upd.push_back(upper ? update(it, b0, k0, k0, k1) : update(it, k1, b1, k0, k1));
+                } else if (upper ? b0 > 0 : b1 < n) {
+                    upd.push_back(upper ? update(it, 0, b0, b0, b1) : update(it, b1, n, b0, b1));
                 }
-            };
-            // Rows are independent within a step: four rows' operands are
-            // loaded before their updates.
-            int i = i0 + L;
-            for (; i + 48 < i1; i += 64) {
-                E fv[4], xv[4];
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    fv[u] = fc[i + 16 * u - r0];
-                    xv[u] = y[i + 16 * u];
-                }
-#pragma unroll
-                for (int u = 0; u < 4; ++u) update(i + 16 * u, fv[u], xv[u]);
             }
-            for (; i < i1; i += 16) update(i, fc[i - r0], y[i]);
+            launch_subst_step(ctx, cplx, upper, diag, upd, lower_divides);
         }
-        // Every lane read x_p above; the divided value goes back only now.
-        if ((UPPER || LDIV) && L == 0) {
-            if constexpr (CPLX) y[p] = make_double2(xk.re, xk.im);
-            else y[p] = xk.re;
-        }
-        __syncwarp();
-    }
-    if (active)
-        for (int p = L; p < n; p += 16) xg[p] = y[p];
 }
 
-template <bool CPLX, bool UPPER, bool LDIV>
-void launch_subst_fused(Context& ctx, const std::vector<SubstFusedDesc>& v, int nmax, int pairs) {
-    static std::atomic<bool> done[64];
-    if (!done[ctx.device].load(std::memory_order_acquire)) {
-        TNS_CUDA(cudaFuncSetAttribute(subst_fused_kernel<CPLX, UPPER, LDIV>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-        done[ctx.device].store(true, std::memory_order_release);
+void substitute(Context& ctx, bool cplx, bool upper, bool lower_divides, const std::vector<SubstItem>& all) {
+    if (wide_batch(ctx, all)) {
+        substitute_wide(ctx, cplx, upper, lower_divides, all);
+        return;
     }
-    const size_t smem = (size_t)(kStageSlots + 2) * nmax * (CPLX ? 16 : 8);
-    subst_fused_kernel<CPLX, UPPER, LDIV><<<dim3(pairs, (unsigned)v.size()), 32, smem, ctx.stream>>>(
-        make_batch(ctx, v), nmax);
-    TNS_CUDA(cudaGetLastError());
-    ctx.kernel_launches++;
-}
-
-void substitute(Context& ctx, bool cplx, bool upper, bool lower_divides, const std::vector<SubstItem>& items) {
-    {
-        // A few complex right-hand sides of orders that fit shared memory: one
-        // launch.
-        int nmax = 0, rmax = 0;
-        bool fits = cplx;
-        for (auto& it : items) {
-            if (it.n == 0 || it.nrhs == 0) continue;
-            nmax = std::max(nmax, it.n);
-            rmax = std::max(rmax, it.nrhs);
-            fits = fits && it.n <= kSubstFusedMaxN && it.nrhs <= kSubstFusedMaxRhs;
-        }
-        if (nmax == 0) return;
-        if (fits) {
-            std::vector<SubstFusedDesc> v;
-            for (auto& it : items)
-                if (it.n > 0 && it.nrhs > 0) v.push_back(SubstFusedDesc{it.f, it.ldf, it.x, it.ldx, it.n, it.nrhs});
-            const int pairs = (rmax + 1) / 2;
-            if (upper) launch_subst_fused<true, true, false>(ctx, v, nmax, pairs);
-            else if (lower_divides) launch_subst_fused<true, false, true>(ctx, v, nmax, pairs);
-            else launch_subst_fused<true, false, false>(ctx, v, nmax, pairs);
-            return;
-        }
+    // Orders whose columns fit shared memory: one launch (subst_cols.cu).
+    std::vector<SubstCols> cols;
+    std::vector<SubstItem> items;
+    for (auto& it : all) {
+        if (it.n <= subst_cols_max_order(cplx)) cols.push_back(SubstCols{it.f, it.ldf, it.x, it.ldx, it.n, it.nrhs, nullptr});
+        else items.push_back(it);
     }
+    subst_cols(ctx, cplx, upper ? LowerKind::kNone : lower_divides ? LowerKind::kDivide : LowerKind::kUnit, upper, cols);
     constexpr int B = kSubstBlock;
     int steps = 0;
     for (auto& it : items)
@@ -1690,6 +1508,39 @@ void getrf_batch(Context& ctx, std::vector<LuItem>& items) {
     }
 }
 
+namespace {
+// The row permutation of every item's interchanges (row k of P B is row perm[k]
+// of B), in one launch into `buf`.
+std::vector<const int*> build_perms(Context& ctx, const std::vector<SolveItem*>& items, DBuf& buf) {
+    size_t total = 0;
+    int maxn = 0;
+    for (auto* it : items) {
+        total += (size_t)it->lu->rows;
+        maxn = std::max(maxn, it->lu->rows);
+    }
+    buf = DBuf(ctx, sizeof(int) * total);
+    std::vector<PermDesc> pd;
+    std::vector<const int*> out;
+    size_t off = 0;
+    for (auto* it : items) {
+        pd.push_back(PermDesc{it->d_piv, it->lu->rows, buf.as<int>() + off});
+        out.push_back(buf.as<int>() + off);
+        off += (size_t)it->lu->rows;
+    }
+    Batch<PermDesc> bp = make_batch(ctx, pd);
+    static std::atomic<bool> configured[64];
+    if (!configured[ctx.device].load(std::memory_order_acquire)) {
+        TNS_CUDA(cudaFuncSetAttribute(build_perm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)(sizeof(int) * 2 * kGatherMaxRows)));
+        configured[ctx.device].store(true, std::memory_order_release);
+    }
+    build_perm_kernel<<<bp.count, 256, sizeof(int) * 2 * (size_t)maxn, ctx.stream>>>(bp);
+    TNS_CUDA(cudaGetLastError());
+    ctx.kernel_launches++;
+    return out;
+}
+}  // namespace
+
 void getrs_batch(Context& ctx, std::vector<SolveItem>& items, bool adjoint) {
     if (items.empty()) return;
     const bool cplx = items[0].lu->cplx;
@@ -1706,52 +1557,50 @@ void getrs_batch(Context& ctx, std::vector<SolveItem>& items, bool adjoint) {
         // the reference's order (Lu.Solve, Lu.cs:336-351; BlockedLu.Solve,
         // BlockedLu.cs:105-118): the result matches the reference bit for bit.
         std::vector<LaswpDesc> swaps;
-        std::vector<SolveItem*> narrow;
+        std::vector<SolveItem*> narrow, fit;
+        std::vector<SubstItem> all;
+        for (auto& it : items)
+            all.push_back(SubstItem{it.lu->p, it.lu->ld(), it.b->p, it.b->ld(), it.lu->rows, it.nrhs});
+        const bool wide = wide_batch(ctx, all);
         for (auto& it : items) {
             int n = it.lu->rows;
             if (n == 0 || it.nrhs == 0) continue;
-            if (it.nrhs < kGatherMaxCols && n <= kGatherMaxRows) narrow.push_back(&it);
+            if (!wide && n <= kGatherMaxRows && n <= subst_cols_max_order(cplx)) fit.push_back(&it);
+            else if (it.nrhs < kGatherMaxCols && n <= kGatherMaxRows) narrow.push_back(&it);
             else swaps.push_back(LaswpDesc{it.b->p, it.b->ld(), 0, it.nrhs, it.d_piv, 0, n, 0});
+        }
+        if (!fit.empty()) {
+            // Columns that fit shared memory: the interchanges as they are
+            // read, then both triangles, in one launch.
+            DBuf perms;
+            std::vector<const int*> perm = build_perms(ctx, fit, perms);
+            std::vector<SubstCols> cols;
+            for (size_t q = 0; q < fit.size(); ++q)
+                cols.push_back(SubstCols{fit[q]->lu->p, fit[q]->lu->ld(), fit[q]->b->p, fit[q]->b->ld(),
+                                         fit[q]->lu->rows, fit[q]->nrhs, perm[q]});
+            subst_cols(ctx, cplx, LowerKind::kUnit, true, cols);
         }
         launch_laswp(ctx, cplx, swaps);
         if (!narrow.empty()) {
-            size_t total = 0;
-            int maxn = 0;
-            for (auto* it : narrow) {
-                total += (size_t)it->lu->rows;
-                maxn = std::max(maxn, it->lu->rows);
-            }
-            DBuf perms(ctx, sizeof(int) * total);
+            DBuf perms;
+            std::vector<const int*> perm = build_perms(ctx, narrow, perms);
             std::vector<DMat> tmp;
             tmp.reserve(narrow.size());
-            std::vector<PermDesc> pd;
             std::vector<GatherDesc> gd;
-            size_t off = 0;
             long long maxe = 0;
-            for (auto* it : narrow) {
+            for (size_t q = 0; q < narrow.size(); ++q) {
+                auto* it = narrow[q];
                 const int n = it->lu->rows;
                 tmp.emplace_back(ctx, it->b->rows, it->b->cols, cplx, "the permuted right-hand sides");
-                pd.push_back(PermDesc{it->d_piv, n, perms.as<int>() + off});
-                gd.push_back(GatherDesc{it->b->p, tmp.back().p, it->b->ld(), n, it->nrhs, perms.as<int>() + off});
-                off += (size_t)n;
+                gd.push_back(GatherDesc{it->b->p, tmp.back().p, it->b->ld(), n, it->nrhs, perm[q]});
                 maxe = std::max(maxe, (long long)n * it->nrhs);
             }
-            Batch<PermDesc> bp = make_batch(ctx, pd);
-            const size_t smem = sizeof(int) * 2 * (size_t)maxn;
-            static bool configured[64] = {};
-            if (!configured[ctx.device]) {
-                TNS_CUDA(cudaFuncSetAttribute(build_perm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              (int)(sizeof(int) * 2 * kGatherMaxRows)));
-                configured[ctx.device] = true;
-            }
-            build_perm_kernel<<<bp.count, 256, smem, ctx.stream>>>(bp);
-            TNS_CUDA(cudaGetLastError());
             Batch<GatherDesc> bg = make_batch(ctx, gd);
             const dim3 grid((unsigned)std::min<long long>((maxe + 255) / 256, ctx.num_sms * 8), bg.count);
             if (cplx) gather_rows_kernel<true><<<grid, 256, 0, ctx.stream>>>(bg);
             else gather_rows_kernel<false><<<grid, 256, 0, ctx.stream>>>(bg);
             TNS_CUDA(cudaGetLastError());
-            ctx.kernel_launches += 2;
+            ctx.kernel_launches++;
             // back into B, only the solve's nrhs columns (contiguous: ld = rows_p)
             for (size_t q = 0; q < narrow.size(); ++q)
                 TNS_CUDA(cudaMemcpyAsync(narrow[q]->b->p, tmp[q].p,
@@ -1760,7 +1609,8 @@ void getrs_batch(Context& ctx, std::vector<SolveItem>& items, bool adjoint) {
         }
         std::vector<SubstItem> subst;
         for (auto& it : items)
-            if (it.lu->rows > 0 && it.nrhs > 0)
+            if (it.lu->rows > 0 && it.nrhs > 0 &&
+                std::none_of(fit.begin(), fit.end(), [&](const SolveItem* f) { return f == &it; }))
                 subst.push_back(SubstItem{it.lu->p, it.lu->ld(), it.b->p, it.b->ld(), it.lu->rows, it.nrhs});
         substitute(ctx, cplx, false, false, subst);  // L, unit diagonal, forward
         substitute(ctx, cplx, true, false, subst);   // U, backward
