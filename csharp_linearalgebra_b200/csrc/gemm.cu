@@ -28,8 +28,9 @@
 //    consecutive rows of column-major C and the epilogue moves 16-byte pairs.
 //  - Persistent CTAs walk a list of problems (grouped GEMM): the same kernel
 //    serves one product, or every matrix of a batch in one launch.
-//  - A single product with fewer tiles than SMs and several KC slabs (1024^3:
-//    64 tiles of 128 x 128, four slabs) is slab-split: every (tile, slab,
+//  - A few products with fewer tiles than SMs and several KC slabs (1024^3:
+//    64 tiles of 128 x 128, four slabs; the products of one Expm at n = 512)
+//    are slab-split: every (tile, slab,
 //    pass) is a unit of its own, writes its raw slab product to a plane, and
 //    a fold kernel adds the planes into C in slab order. Each slab's
 //    accumulation starts from zero in both forms, so the split changes which
@@ -58,12 +59,12 @@
 
 namespace tns {
 
-template <bool CPLX, int WARPS_M, int WARPS_N, int STAGES_>
+template <bool CPLX, int WARPS_M, int WARPS_N, int STAGES_, int WN_ = CPLX ? 32 : 64>
 struct GemmCfg {
     static constexpr bool kComplex = CPLX;
     static constexpr int ESZ = CPLX ? 16 : 8;  // bytes per element
     static constexpr int WM = 32;              // C rows per warp = 4 mma-N fragments of 8
-    static constexpr int WN = CPLX ? 32 : 64;  // C columns per warp, mma-M fragments of 16
+    static constexpr int WN = WN_;             // C columns per warp, mma-M fragments of 16
     static constexpr int MF = WM / 8;
     static constexpr int NF = WN / 16;
     static constexpr int BM = WARPS_M * WM;
@@ -583,7 +584,10 @@ __global__ void __launch_bounds__(256) slab_fold_kernel(const __grid_constant__ 
 namespace {
 
 using RealBig = GemmCfg<false, 4, 2, 4>;    // 128 x 128 tiles, 8 math warps
-using RealSmall = GemmCfg<false, 2, 1, 4>;  // 64 x 64 tiles, 2 math warps
+// 64 x 64 tiles, 4 math warps, one on each SM sub-partition: with two of 32 x 64
+// a tile's 256-deep slab took 17 us on half of an SM's tensor pipes, and the 35
+// products of a real gradient at n = 600 1.49 ms against 0.93.
+using RealSmall = GemmCfg<false, 2, 2, 4, 32>;
 using CplxBig = GemmCfg<true, 4, 2, 3>;     // 128 x 64 tiles, 8 math warps
 using CplxSmall = GemmCfg<true, 2, 2, 4>;   // 64 x 64 tiles, 4 math warps
 
@@ -722,38 +726,53 @@ namespace {
 
 // Slab planes of a slab-split product stay below this size.
 constexpr size_t kSlabPlaneBytes = size_t(512) << 20;
+// Products split in one launch (each is folded by a launch of its own).
+constexpr size_t kSlabSplitProblems = 4;
 
-// One product whose tiles leave SMs idle and whose K spans several KC slabs:
-// each tile's slabs (and passes) run as separate units, so more CTAs work at
-// once, each unit's raw slab product goes to its own plane, and a fold kernel
-// adds the slabs into C in slab order with the operations the unsplit kernel
-// applies at each slab end (the same bits). False when the split does not
-// apply.
+// Products whose tiles leave SMs idle and some of whose K span several KC
+// slabs: each tile's slabs (and passes) run as separate units, so more CTAs
+// work at once, each unit's raw slab product goes to its own plane, and a fold
+// kernel adds the slabs into C in slab order with the operations the unsplit
+// kernel applies at each slab end (the same bits). False when the split does
+// not apply.
 template <class Big, class Small>
-bool slab_split_launch(Context& ctx, const GemmProblem& p0, long long tiles_big) {
+bool slab_split_launch(Context& ctx, const std::vector<GemmProblem>& work, long long tiles_big) {
     constexpr bool CPLX = Big::kComplex;
     constexpr int passes = CPLX ? 2 : 1;
-    const int slabs = (p0.K + p0.kc - 1) / p0.kc;
-    const size_t bytes = (size_t)passes * slabs * p0.M * p0.N * Big::ESZ;
-    if (slabs < 2 || tiles_big >= ctx.num_sms || bytes > kSlabPlaneBytes) return false;
+    if (tiles_big >= ctx.num_sms) return false;
+    size_t bytes = 0;
+    long long units_big = 0;
+    int most = 0;
+    for (auto& p : work) {
+        const int slabs = (p.K + p.kc - 1) / p.kc;
+        most = std::max(most, slabs);
+        bytes += (size_t)passes * slabs * p.M * p.N * Big::ESZ;
+        units_big += (long long)((p.M + Big::BM - 1) / Big::BM) * ((p.N + Big::BN - 1) / Big::BN) * slabs * passes;
+    }
+    if (most < 2 || bytes > kSlabPlaneBytes) return false;
     DBuf planes(ctx, bytes);
-    GemmProblem p = p0;
-    p.S = planes.p;
-    p.slabs = slabs;
-    p.W = nullptr;
-    p.ldw = 0;
-    std::vector<GemmProblem> v{p};
+    std::vector<GemmProblem> v = work;
+    size_t at = 0;
+    for (auto& p : v) {
+        p.slabs = (p.K + p.kc - 1) / p.kc;
+        p.S = planes.as<char>() + at;
+        p.W = nullptr;
+        p.ldw = 0;
+        at += (size_t)passes * p.slabs * p.M * p.N * Big::ESZ;  // a multiple of 16: M is even
+    }
     auto fold = [&] {
-        slab_fold_kernel<CPLX><<<dim3((p.M + 255) / 256, p.N), 256, 0, ctx.stream>>>(p);
-        TNS_CUDA(cudaGetLastError());
-        ctx.kernel_launches++;
+        for (auto& p : v) {
+            slab_fold_kernel<CPLX><<<dim3((p.M + 255) / 256, p.N), 256, 0, ctx.stream>>>(p);
+            TNS_CUDA(cudaGetLastError());
+            ctx.kernel_launches++;
+        }
     };
-    if (tiles_big * slabs * passes >= ctx.num_sms) launch_cfg<Big, true>(ctx, v, fold);
+    if (units_big >= ctx.num_sms) launch_cfg<Big, true>(ctx, v, fold);
     else launch_cfg<Small, true>(ctx, v, fold);
     return true;
 }
 
-void gemm_run(Context& ctx, std::vector<GemmProblem>& probs, bool cplx, bool slab_split) {
+void gemm_run(Context& ctx, std::vector<GemmProblem>& probs, bool cplx) {
     std::vector<GemmProblem> work;
     work.reserve(probs.size());
     for (auto& p0 : probs) {
@@ -782,9 +801,10 @@ void gemm_run(Context& ctx, std::vector<GemmProblem>& probs, bool cplx, bool sla
         depth = std::max(depth, p.K);
         if (p.beta_re != 0.0 || p.beta_im != 0.0) overwrite = false;
     }
-    if (slab_split && work.size() == 1 &&
-        (cplx ? slab_split_launch<CplxBig, CplxSmall>(ctx, work[0], tiles)
-              : slab_split_launch<RealBig, RealSmall>(ctx, work[0], tiles)))
+    // Not in a batch worker: the other workers' launches fill the idle SMs.
+    if (!ctx.concurrent && work.size() <= kSlabSplitProblems &&
+        (cplx ? slab_split_launch<CplxBig, CplxSmall>(ctx, work, tiles)
+              : slab_split_launch<RealBig, RealSmall>(ctx, work, tiles)))
         return;
     std::vector<DBuf> scratch;
     scratch.reserve(work.size());
@@ -819,13 +839,11 @@ void gemm_run(Context& ctx, std::vector<GemmProblem>& probs, bool cplx, bool sla
 
 }  // namespace
 
-void gemm_grouped(Context& ctx, std::vector<GemmProblem>& probs, bool cplx) { gemm_run(ctx, probs, cplx, false); }
+void gemm_grouped(Context& ctx, std::vector<GemmProblem>& probs, bool cplx) { gemm_run(ctx, probs, cplx); }
 
-// One product through the public entry points: slab-split when its tiles
-// alone would leave SMs idle.
 void gemm(Context& ctx, const GemmProblem& p, bool cplx) {
     std::vector<GemmProblem> v{p};
-    gemm_run(ctx, v, cplx, true);
+    gemm_run(ctx, v, cplx);
 }
 
 namespace {
