@@ -472,8 +472,8 @@ void launch_panel(Context& ctx, std::vector<PanelDesc>& v, bool adjoint) {
     if (nmax == 0) return;
     Batch<PanelDesc> b = make_batch(ctx, v);
     if (!adjoint) {
-        // Narrow panels (the estimator's two or four columns): one thread per
-        // (row, column), twice or four times the threads of one per row.
+        // Panels of up to four columns: one thread per (row, column), four
+        // times the threads of one per row.
         constexpr int TPR = TMAX <= 4 ? TMAX : 1;
         dim3 grid((nmax + 128 / TPR - 1) / (128 / TPR), b.count);
         panel_apply_kernel<TMAX, CPLX, TPR><<<grid, 128, 0, ctx.stream>>>(b);
@@ -660,10 +660,13 @@ std::vector<double> abs_power_batch(Context& ctx, const std::vector<const DMat*>
     if (cplx) moduli_kernel<true><<<g0, kThreads, 0, ctx.stream>>>(bc);
     else moduli_kernel<false><<<g0, kThreads, 0, ctx.stream>>>(bc);
     ctx.kernel_launches++;
-    dim3 g1((nmax + 32 * kChainWarps - 1) / (32 * kChainWarps), bc.count);
-    for (int step = 0; step < p; ++step) {
-        abs_power_step_kernel<<<g1, 32 * kChainWarps, 0, ctx.stream>>>(bc, step & 1);
-        ctx.kernel_launches++;
+    if (!abs_power_chains(ctx, chains, p)) {
+        // Orders whose row vector does not fit shared memory: a launch per pass.
+        dim3 g1((nmax + 32 * kChainWarps - 1) / (32 * kChainWarps), bc.count);
+        for (int step = 0; step < p; ++step) {
+            abs_power_step_kernel<<<g1, 32 * kChainWarps, 0, ctx.stream>>>(bc, step & 1);
+            ctx.kernel_launches++;
+        }
     }
     Batch<SumDesc> bf = make_batch(ctx, folds);
     max_fold_kernel<<<bf.count, 256, 0, ctx.stream>>>(bf);
@@ -685,14 +688,16 @@ void panel_product_batch(Context& ctx, std::vector<PanelDesc>& v, bool cplx, boo
     int tmax = 0;
     for (auto& d : v) tmax = std::max(tmax, d.t);
     if (tmax > 16) fail(TNS_E_ARGUMENT, "internal panel product wider than 16 columns");
+    if (tmax <= 2) {
+        narrow_products(ctx, v, cplx, adjoint);
+        return;
+    }
     if (cplx) {
-        if (tmax <= 2) launch_panel<2, true>(ctx, v, adjoint);
-        else if (tmax <= 4) launch_panel<4, true>(ctx, v, adjoint);
+        if (tmax <= 4) launch_panel<4, true>(ctx, v, adjoint);
         else if (tmax <= 8) launch_panel<8, true>(ctx, v, adjoint);
         else launch_panel<16, true>(ctx, v, adjoint);
     } else {
-        if (tmax <= 2) launch_panel<2, false>(ctx, v, adjoint);
-        else if (tmax <= 4) launch_panel<4, false>(ctx, v, adjoint);
+        if (tmax <= 4) launch_panel<4, false>(ctx, v, adjoint);
         else if (tmax <= 8) launch_panel<8, false>(ctx, v, adjoint);
         else launch_panel<16, false>(ctx, v, adjoint);
     }

@@ -283,6 +283,11 @@ std::vector<double> norm1_batch(Context& ctx, const std::vector<const DMat*>& ma
 std::vector<double> norminf_batch(Context& ctx, const std::vector<const DMat*>& mats);
 std::vector<double> abs_power_batch(Context& ctx, const std::vector<const DMat*>& mats, int p);
 void panel_product_batch(Context& ctx, std::vector<PanelDesc>& v, bool cplx, bool adjoint);
+// estimate.cu: the same for panels of one or two columns over library-owned
+// (zero-padded) matrices, and all passes of the ell chains over the moduli in
+// one launch (false, nothing done, when a row vector does not fit shared memory).
+void narrow_products(Context& ctx, std::vector<PanelDesc>& v, bool cplx, bool adjoint);
+bool abs_power_chains(Context& ctx, const std::vector<ChainDesc>& v, int passes);
 
 // ---- elementwise and reductions (blas1.cu) ---------------------------------
 void scale_inplace(Context& ctx, void* c, int m, int n, int ldc, bool cplx, double beta_re, double beta_im);
