@@ -28,6 +28,7 @@
 #include "device_util.cuh"
 #include "lu_panel.h"
 #include "subst_cols.h"
+#include "subst_left.h"
 #include "tns_internal.h"
 
 #include <algorithm>
@@ -803,9 +804,13 @@ __global__ void fill_int_kernel(int* p, int count, int v) {
 
 // P B for a solve with few right-hand sides: laswp gives each column one
 // thread and n sequential swaps, which leaves the GPU idle when B is narrow.
-// Instead one CTA per item replays the swaps on an index array in shared
-// memory (row k of P B is row perm[k] of B), and a gather moves every row
-// once. The result is the same values in the same places.
+// Instead one CTA per item turns the swaps into a permutation (row k of P B is
+// row perm[k] of B), applied where the rows are next read or written. Swap k
+// brings to position k, for good, what its partner p_k >= k holds: the values
+// that the latest earlier swap with the same partner put there, which are those
+// that swap's own position held, and so on back to a row not yet touched. Those
+// references are formed 32 swaps at a time and followed by pointer jumping,
+// where replaying the swaps one by one took 41 us at n = 512.
 struct PermDesc {
     const int* piv;
     int n;
@@ -813,24 +818,51 @@ struct PermDesc {
 };
 __global__ void build_perm_kernel(const __grid_constant__ Batch<PermDesc> b) {
     const PermDesc& d = batch_item(b, blockIdx.x);
-    extern __shared__ int sp[];  // perm [n], pivots [n]
-    int* pv = sp + d.n;
-    for (int i = threadIdx.x; i < d.n; i += blockDim.x) {
-        sp[i] = i;
-        pv[i] = d.piv[i];
+    extern __shared__ int sp[];  // last [n], root [n]
+    const int n = d.n;
+    int* last = sp;
+    int* root = sp + n;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) last[i] = -1;
+    __syncthreads();
+    // The latest earlier swap with the same partner, swaps in order, a warp at a
+    // time: within 32 swaps by matching, across them through last[].
+    if (threadIdx.x < 32) {
+        const int lane = threadIdx.x;
+        int p = lane < n ? d.piv[lane] : 0;
+        for (int k0 = 0; k0 < n; k0 += 32) {
+            const int k = k0 + lane;
+            const int ahead = k + 32 < n ? d.piv[k + 32] : 0;
+            const bool real = k < n && p != k;
+            const unsigned same = __match_any_sync(0xffffffffu, real ? p : -1 - lane);
+            const unsigned before = same & ((1u << lane) - 1);
+            if (real) d.perm[k] = before ? k0 + 31 - __clz(before) : last[p];
+            else if (k < n) d.perm[k] = -1;
+            __syncwarp();
+            if (real && (same >> lane) == 1u) last[p] = k;  // the latest of its partner
+            __syncwarp();
+            p = ahead;
+        }
     }
     __syncthreads();
-    if (threadIdx.x == 0)
-        for (int k = 0; k < d.n; ++k) {
-            const int p = pv[k];
-            if (p != k) {
-                const int t = sp[k];
-                sp[k] = sp[p];
-                sp[p] = t;
+    // root[k]: the row whose values position k holds just before swap k: its own,
+    // or those that the latest swap with partner k brought.
+    for (int i = threadIdx.x; i < n; i += blockDim.x) root[i] = last[i] < 0 ? i : last[i];
+    __syncthreads();
+    for (;;) {
+        int changed = 0;
+        for (int i = threadIdx.x; i < n; i += blockDim.x) {
+            const int r = root[i], rr = root[r];
+            if (rr != r) {
+                root[i] = rr;  // an ancestor either way: concurrent steps only shorten the way
+                changed = 1;
             }
         }
-    __syncthreads();
-    for (int i = threadIdx.x; i < d.n; i += blockDim.x) d.perm[i] = sp[i];
+        if (!__syncthreads_or(changed)) break;
+    }
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        const int p = d.piv[i], prev = d.perm[i];
+        d.perm[i] = p == i ? root[i] : prev >= 0 ? root[prev] : p;
+    }
 }
 struct GatherDesc {
     const double* src;
@@ -1047,12 +1079,6 @@ struct SubstItem {
     double* x;
     int ldx, n, nrhs;
 };
-// The staged left-looking kernels below copy the factor column of step s +
-// kStageAhead while step s runs, into a ring of kStageSlots columns: far
-// enough ahead that the copies' latency is hidden.
-constexpr int kStageSlots = 6;
-constexpr int kStageAhead = kStageSlots - 1;
-
 // A batch with many more columns than the GPU takes at once in the one-launch
 // solve (ctas: its CTAs of eight columns, each keeping a whole SM): there the
 // columns alone fill the GPU, and what counts is FP64 work per column. So the
@@ -1208,13 +1234,16 @@ __global__ void __launch_bounds__(64) left_subst_cplx_unit_back_kernel(const dou
 }
 
 // The same two solves with the right-hand sides and the factor in shared
-// memory, for the orders that fit: one warp per pair of right-hand sides (a
+// memory, for the orders that fit and more right-hand sides than
+// subst_left.cu's kernels run at once: one warp per pair of right-hand sides (a
 // half-warp each, both on the same row at each step), the pair's columns kept
 // in shared memory, and the factor column a step reads (with its diagonal)
 // copied in by cp.async kStageAhead steps ahead into a ring of kStageSlots. A
 // step then reads nothing from global memory, and its sums are the kernels' above,
 // term for term. Complex: the products conj(f_ki) x[k] of a row are formed by
 // the half-warp, then one lane subtracts them in ascending k.
+constexpr int kStageSlots = 6;
+constexpr int kStageAhead = kStageSlots - 1;
 constexpr int kLeftRealMaxN = 3200;  // 6 slots + 2 columns of doubles: 200 KB
 constexpr int kLeftCplxMaxN = 1280;  // 6 slots + 2 columns + 2 product rows of complex: 200 KB
 
@@ -1350,11 +1379,19 @@ void allow_left_smem(int device) {
     done[device].store(true, std::memory_order_release);
 }
 
-// One left-looking solve (see left_subst_real_kernel): real forward U^T
-// (unit = false) or backward L^T (unit or not); complex: backward L^H, unit.
+// One left-looking solve: real forward U^T (unit = false) or backward L^T (unit
+// or not); complex: backward L^H, unit. Orders whose products fit shared memory
+// run on subst_left.cu's kernels.
 void left_substitute(Context& ctx, bool cplx, bool forward, bool unit, const double* f, int ldf, double* x, int ldx,
                      int n, int nrhs) {
     if (n == 0 || nrhs == 0) return;
+    if (cplx ? forward || !unit : forward && unit) fail(TNS_E_ARGUMENT, "internal: no such left-looking solve");
+    if (left_solve_takes(ctx, cplx, n, nrhs)) {
+        const LeftSolve s{f, ldf, x, ldx, n, nrhs, nullptr};
+        if (cplx) left_solve_cplx(ctx, s);
+        else left_solve_real(ctx, forward, forward ? LowerKind::kNone : unit ? LowerKind::kUnit : LowerKind::kDivide, s);
+        return;
+    }
     const unsigned pairs = (unsigned)((nrhs + 1) / 2);
     if (!cplx && n <= kLeftRealMaxN) {
         const size_t smem = sizeof(double) * (size_t)(kStageSlots + 2) * n;
@@ -1364,11 +1401,9 @@ void left_substitute(Context& ctx, bool cplx, bool forward, bool unit, const dou
         } else if (!forward && unit) {
             allow_left_smem<left_subst_real_staged_kernel<false, true>>(ctx.device);
             left_subst_real_staged_kernel<false, true><<<pairs, 32, smem, ctx.stream>>>(f, ldf, x, ldx, n, nrhs);
-        } else if (!forward && !unit) {
+        } else {
             allow_left_smem<left_subst_real_staged_kernel<false, false>>(ctx.device);
             left_subst_real_staged_kernel<false, false><<<pairs, 32, smem, ctx.stream>>>(f, ldf, x, ldx, n, nrhs);
-        } else {
-            fail(TNS_E_ARGUMENT, "internal: no unit forward transposed solve");
         }
         TNS_CUDA(cudaGetLastError());
         ctx.kernel_launches++;
@@ -1384,12 +1419,10 @@ void left_substitute(Context& ctx, bool cplx, bool forward, bool unit, const dou
     }
     if (!cplx) {
         const unsigned grid = (unsigned)((nrhs * 16 + 127) / 128);
-        if (forward && !unit) left_subst_real_kernel<true, false><<<grid, 128, 0, ctx.stream>>>(f, ldf, x, ldx, n, nrhs);
-        else if (!forward && unit) left_subst_real_kernel<false, true><<<grid, 128, 0, ctx.stream>>>(f, ldf, x, ldx, n, nrhs);
-        else if (!forward && !unit) left_subst_real_kernel<false, false><<<grid, 128, 0, ctx.stream>>>(f, ldf, x, ldx, n, nrhs);
-        else fail(TNS_E_ARGUMENT, "internal: no unit forward transposed solve");
+        if (forward) left_subst_real_kernel<true, false><<<grid, 128, 0, ctx.stream>>>(f, ldf, x, ldx, n, nrhs);
+        else if (unit) left_subst_real_kernel<false, true><<<grid, 128, 0, ctx.stream>>>(f, ldf, x, ldx, n, nrhs);
+        else left_subst_real_kernel<false, false><<<grid, 128, 0, ctx.stream>>>(f, ldf, x, ldx, n, nrhs);
     } else {
-        if (forward || !unit) fail(TNS_E_ARGUMENT, "internal: complex left-looking solves are backward and unit");
         left_subst_cplx_unit_back_kernel<<<(unsigned)((nrhs + 63) / 64), 64, 0, ctx.stream>>>(f, ldf, x, ldx, n, nrhs);
     }
     TNS_CUDA(cudaGetLastError());
@@ -1619,32 +1652,45 @@ void getrs_batch(Context& ctx, std::vector<SolveItem>& items, bool adjoint) {
     // The adjoint in the reference's order (Lu.SolveTransposed, Lu.cs:364-378;
     // BlockedLu.SolveAdjoint, BlockedLu.cs:130-141): U^H forward, then L^H
     // backward, then the interchanges undone.
+    // Where the left-looking kernels take the order, they also undo the
+    // interchanges, as they write the solution.
+    std::vector<SolveItem*> fit;
+    for (auto& it : items)
+        if (it.nrhs > 0 && it.lu->rows > 0 && it.lu->rows <= kGatherMaxRows &&
+            left_solve_takes(ctx, cplx, it.lu->rows, it.nrhs))
+            fit.push_back(&it);
+    DBuf perms;
+    std::vector<const int*> perm;
+    if (!fit.empty()) perm = build_perms(ctx, fit, perms);
+    std::vector<LaswpDesc> swaps;
+    size_t next_fit = 0;
     for (size_t q = 0; q < items.size(); ++q) {
         auto& it = items[q];
         const int n = it.lu->rows;
         if (n == 0 || it.nrhs == 0) continue;
+        const bool fits = next_fit < fit.size() && fit[next_fit] == &it;
+        const LeftSolve s{it.lu->p, it.lu->ld(), it.b->p, it.b->ld(), n, it.nrhs, fits ? perm[next_fit] : nullptr};
+        if (fits) ++next_fit;
+        else swaps.push_back(LaswpDesc{it.b->p, it.b->ld(), 0, it.nrhs, it.d_piv, 0, n, 1});
         if (!cplx) {
             // Both by inner products in ColumnOps.Dot's order.
-            left_substitute(ctx, false, true, false, it.lu->p, it.lu->ld(), it.b->p, it.b->ld(), n, it.nrhs);
-            left_substitute(ctx, false, false, true, it.lu->p, it.lu->ld(), it.b->p, it.b->ld(), n, it.nrhs);
+            if (fits) {
+                left_solve_real(ctx, true, LowerKind::kUnit, s);
+            } else {
+                left_substitute(ctx, false, true, false, s.f, s.ldf, s.x, s.ldx, n, s.nrhs);
+                left_substitute(ctx, false, false, true, s.f, s.ldf, s.x, s.ldx, n, s.nrhs);
+            }
         } else {
             // U^H: its sums run in ascending k, which a right-looking sweep over
             // the conjugate transpose reproduces; L^H: ascending k inside a
             // backward sweep, one inner product per row.
-            std::vector<SubstItem> fwd{SubstItem{herm[q].p, herm[q].ld(), it.b->p, it.b->ld(), n, it.nrhs}};
+            std::vector<SubstItem> fwd{SubstItem{herm[q].p, herm[q].ld(), s.x, s.ldx, n, s.nrhs}};
             substitute(ctx, true, false, true, fwd);
-            left_substitute(ctx, true, false, true, it.lu->p, it.lu->ld(), it.b->p, it.b->ld(), n, it.nrhs);
+            if (fits) left_solve_cplx(ctx, s);
+            else left_substitute(ctx, true, false, true, s.f, s.ldf, s.x, s.ldx, n, s.nrhs);
         }
     }
-    if (adjoint) {
-        std::vector<LaswpDesc> swaps;
-        for (auto& it : items) {
-            int n = it.lu->rows;
-            if (n == 0 || it.nrhs == 0) continue;
-            swaps.push_back(LaswpDesc{it.b->p, it.b->ld(), 0, it.nrhs, it.d_piv, 0, n, 1});
-        }
-        launch_laswp(ctx, cplx, swaps);
-    }
+    launch_laswp(ctx, cplx, swaps);
 }
 
 LuResult getrf(Context& ctx, DMat& a, int m, int n, int nb, int* d_piv) {
