@@ -7,8 +7,9 @@
 //   1. panel factorization (one CTA per matrix; pivot = first index of the
 //      largest |a|, or |Re|+|Im| for complex; reciprocal multiply unless
 //      |pivot| < SafeMin; rank-1 updates y + (-m)*x with two roundings),
-//   2. the panel's row interchanges applied to the columns either side,
-//   3. U12 := L11^-1 A12 (one warp per column, the reference's update order),
+//   2. the panel's row interchanges applied to the columns either side, and
+//   3. U12 := L11^-1 A12 in the same pass (lu_panel.cu, one warp per column, the
+//      reference's update order),
 //   4. A22 := A22 - A21*U12 on the DMMA GEMM (bit-identical to the
 //      reference's product, gemm.cu).
 // Every step's arithmetic is the reference's, so the factors and pivots match
@@ -483,14 +484,9 @@ __global__ void laswp_kernel(const __grid_constant__ Batch<LaswpDesc> b) {
     }
 }
 
-// Triangular block solves, one warp per right-hand side column, w <= 64.
-//  kind 0: B := L^-1 B for the unit lower L at t, with the reference's order
-//          (x[i] += (-x[p]) * L[i, p] for p = 0..w-2, columns with x[p] == 0
-//          skipped; Triangular.SolveLowerUnit, Triangular.cs:26-57, and the
-//          complex BlockedLu.cs:312-327).
-//  kind 1: X := T^-1 X for the diagonal block of the blocked solves: lower or
-//          upper, unit or not, optionally the conjugate transpose of the stored
-//          block.
+// Triangular block solves, one warp per right-hand side column, w <= 64:
+// X := T^-1 X for the diagonal block of the blocked solves, lower or upper,
+// unit or not, optionally the conjugate transpose of the stored block.
 struct TrsmDesc {
     const double* t;
     int ldt;
@@ -499,7 +495,7 @@ struct TrsmDesc {
     int lower, unit, conj;
 };
 
-template <bool CPLX, int KIND>
+template <bool CPLX>
 __global__ void trsm_kernel(const __grid_constant__ Batch<TrsmDesc> bt) {
     const TrsmDesc& d = batch_item(bt, blockIdx.y);
     constexpr int ES = CPLX ? 2 : 1;
@@ -541,12 +537,11 @@ __global__ void trsm_kernel(const __grid_constant__ Batch<TrsmDesc> bt) {
             v[h].re = i < w ? x[(size_t)i * ES] : 0.0;
             v[h].im = (CPLX && i < w) ? x[(size_t)i * ES + 1] : 0.0;
         }
-        const int steps = KIND == 0 ? w - 1 : w;
-        for (int s = 0; s < steps; ++s) {
-            const bool lower = KIND == 0 ? true : d.lower != 0;
+        for (int s = 0; s < w; ++s) {
+            const bool lower = d.lower != 0;
             int p = lower ? s : w - 1 - s;
             int h = p >> 5, src = p & 31;
-            if (KIND == 1 && !d.unit) {
+            if (!d.unit) {
                 if (lane == src) {
                     if (!CPLX) {
                         v[h].re = __ddiv_rn(v[h].re, sT[(size_t)p * w + p]);
@@ -558,7 +553,6 @@ __global__ void trsm_kernel(const __grid_constant__ Batch<TrsmDesc> bt) {
             }
             double vr = __shfl_sync(0xffffffffu, v[h].re, src);
             double vi = CPLX ? __shfl_sync(0xffffffffu, v[h].im, src) : 0.0;
-            if (KIND == 0 && vr == 0.0 && vi == 0.0) continue;
             for (int q = 0; q < 2; ++q) {
                 int i = lane + 32 * q;
                 bool beyond = lower ? (i > p) : (i < p);
@@ -962,38 +956,33 @@ void launch_laswp(Context& ctx, bool cplx, std::vector<LaswpDesc>& v) {
     ctx.kernel_launches++;
 }
 
-template <bool CPLX, int KIND>
+template <bool CPLX>
 void launch_trsm_t(Context& ctx, std::vector<TrsmDesc>& live, int maxcols) {
     // The 64 x 64 complex block needs 64 KB of dynamic shared memory, above
     // the default 48 KB; the attribute is per kernel instance.
-    TNS_CUDA(cudaFuncSetAttribute(trsm_kernel<CPLX, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 64 * 16));
+    TNS_CUDA(cudaFuncSetAttribute(trsm_kernel<CPLX>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 64 * 16));
     Batch<TrsmDesc> b = make_batch(ctx, live);
     const int threads = 256, warps = threads / 32;
     int per_item = std::max(1, std::min((maxcols + warps - 1) / warps, std::max(1, ctx.num_sms * 4 / (int)live.size())));
     int wmax = 0;
     for (auto& d : live) wmax = std::max(wmax, d.w);
     size_t smem = (size_t)wmax * wmax * (CPLX ? 16 : 8);
-    trsm_kernel<CPLX, KIND><<<dim3(per_item, b.count), threads, smem, ctx.stream>>>(b);
+    trsm_kernel<CPLX><<<dim3(per_item, b.count), threads, smem, ctx.stream>>>(b);
     TNS_CUDA(cudaGetLastError());
     ctx.kernel_launches++;
 }
 
-void launch_trsm(Context& ctx, bool cplx, int kind, std::vector<TrsmDesc>& v) {
+void launch_trsm(Context& ctx, bool cplx, std::vector<TrsmDesc>& v) {
     std::vector<TrsmDesc> live;
     int maxcols = 0;
     for (auto& d : v)
-        if (d.ncols > 0 && d.w > (kind == 0 ? 1 : 0)) {
+        if (d.ncols > 0 && d.w > 0) {
             live.push_back(d);
             maxcols = std::max(maxcols, d.ncols);
         }
     if (live.empty()) return;
-    if (cplx) {
-        if (kind == 0) launch_trsm_t<true, 0>(ctx, live, maxcols);
-        else launch_trsm_t<true, 1>(ctx, live, maxcols);
-    } else {
-        if (kind == 0) launch_trsm_t<false, 0>(ctx, live, maxcols);
-        else launch_trsm_t<false, 1>(ctx, live, maxcols);
-    }
+    if (cplx) launch_trsm_t<true>(ctx, live, maxcols);
+    else launch_trsm_t<false>(ctx, live, maxcols);
 }
 
 // One block step of the substitution for every item of a batch: the
@@ -1035,16 +1024,15 @@ void launch_subst_step(Context& ctx, bool cplx, bool upper, std::vector<SubstDia
 // rank-1 updates would: the interchanges, the rows of the left half's pivots
 // (a unit lower solve), and every row below, each element's updates in order
 // with two roundings (the substitution kernels, whose step is the same
-// x + (-u) l). The right half's interchanges of the left half's columns are
-// added to `swaps`, which the caller launches next. Taller panels keep the
-// kernels above.
-void factor_panels(Context& ctx, bool cplx, std::vector<PanelFactorDesc>& v, std::vector<LaswpDesc>& swaps) {
+// x + (-u) l); the right half carries the left half's rows along. Taller
+// panels keep the kernels above.
+void factor_panels(Context& ctx, bool cplx, std::vector<PanelFactorDesc>& v) {
     std::vector<PanelFactorDesc> rows, tall;
     for (auto& p : v) (p.m - p.r0 <= row_panel_max_rows(cplx) ? rows : tall).push_back(p);
     constexpr int W = kRowPanelWidth;
     std::vector<PanelFactorDesc> left, right;
-    std::vector<LaswpDesc> inner;
-    std::vector<SubstDiagDesc> diag;
+    std::vector<PanelRowsDesc> inner;
+    std::vector<SubstDiagDesc> none;
     std::vector<SubstUpdateDesc> upd;
     const size_t es = cplx ? 2 : 1;
     for (auto& p : rows) {
@@ -1054,16 +1042,14 @@ void factor_panels(Context& ctx, bool cplx, std::vector<PanelFactorDesc>& v, std
         if (p.w <= W) continue;
         const int M = p.m - p.r0, done = std::min(M, W), cols = p.w - W, c0 = p.r0 + W;
         double* x = p.a + (size_t)c0 * p.ld * es;
-        inner.push_back(LaswpDesc{p.a, p.ld, c0, c0 + cols, p.piv, p.r0, p.r0 + done, 0});
-        diag.push_back(SubstDiagDesc{p.a, p.ld, x, p.ld, cols, p.r0, done});
+        inner.push_back(PanelRowsDesc{p.a, p.ld, c0, c0 + cols, p.piv, p.r0, done, 1, 1, 0});
         if (M <= W) continue;
         upd.push_back(SubstUpdateDesc{p.a, p.ld, x, p.ld, cols, p.r0 + W, p.m, p.r0, p.r0 + W, (M - W + 63) / 64, 0});
-        right.push_back(PanelFactorDesc{p.a, p.ld, p.m, p.r0 + W, cols, p.piv, p.singular});
-        swaps.push_back(LaswpDesc{p.a, p.ld, p.r0, p.r0 + W, p.piv, p.r0 + W, p.r0 + std::min(M, p.w), 0});
+        right.push_back(PanelFactorDesc{p.a, p.ld, p.m, p.r0 + W, cols, p.piv, p.singular, W});
     }
     launch_row_panels(ctx, cplx, left);
-    launch_laswp(ctx, cplx, inner);
-    launch_subst_step(ctx, cplx, false, diag, upd);
+    launch_panel_rows(ctx, cplx, inner);
+    launch_subst_step(ctx, cplx, false, none, upd);
     launch_row_panels(ctx, cplx, right);
     launch_tall_panels(ctx, cplx, tall);
 }
@@ -1473,8 +1459,7 @@ void getrf_batch(Context& ctx, std::vector<LuItem>& items) {
     }
     for (int k = 0; k < max_steps; ++k) {
         std::vector<PanelFactorDesc> panels;
-        std::vector<LaswpDesc> swaps;
-        std::vector<TrsmDesc> trsms;
+        std::vector<PanelRowsDesc> rows;  // interchanges, and U12 to the right
         std::vector<GemmProblem> gemms;
         for (auto& it : items) {
             DMat& a = *it.a;
@@ -1482,17 +1467,16 @@ void getrf_batch(Context& ctx, std::vector<LuItem>& items) {
             const int limit = std::min(m, n);
             if (limit == 0) continue;
             if (it.nb >= limit && n <= 64) {
-                if (k == 0) panels.push_back(PanelFactorDesc{a.p, ld, m, 0, n, it.d_piv, it.d_sing});
+                if (k == 0) panels.push_back(PanelFactorDesc{a.p, ld, m, 0, n, it.d_piv, it.d_sing, 0});
                 continue;
             }
             const int jb = k * it.nb;
             if (jb >= limit) continue;
             const int w = std::min(it.nb, limit - jb);
-            panels.push_back(PanelFactorDesc{a.p, ld, m, jb, w, it.d_piv, it.d_sing});
-            swaps.push_back(LaswpDesc{a.p, ld, 0, jb, it.d_piv, jb, jb + w, 0});
+            panels.push_back(PanelFactorDesc{a.p, ld, m, jb, w, it.d_piv, it.d_sing, 0});
+            rows.push_back(PanelRowsDesc{a.p, ld, 0, jb, it.d_piv, jb, w, 1, 0, 0});
             if (jb + w >= n) continue;
-            swaps.push_back(LaswpDesc{a.p, ld, jb + w, n, it.d_piv, jb, jb + w, 0});
-            trsms.push_back(TrsmDesc{a.p + off(a, jb, jb), ld, a.p + off(a, jb, jb + w), ld, w, n - jb - w, 1, 1, 0});
+            rows.push_back(PanelRowsDesc{a.p, ld, jb + w, n, it.d_piv, jb, w, 1, 1, 0});
             if (jb + w >= m) continue;
             GemmProblem p{};
             p.A = a.p + off(a, jb + w, jb);
@@ -1508,12 +1492,20 @@ void getrf_batch(Context& ctx, std::vector<LuItem>& items) {
             gemms.push_back(p);
         }
         if (timed) mark();
-        factor_panels(ctx, cplx, panels, swaps);
-        if (timed) mark();
-        launch_laswp(ctx, cplx, swaps);
-        if (timed) mark();
-        launch_trsm(ctx, cplx, 0, trsms);
-        if (timed) mark();
+        factor_panels(ctx, cplx, panels);
+        if (timed) {
+            // The phases apart: the interchanges, then U12.
+            std::vector<PanelRowsDesc> swaps = rows, solves = rows;
+            for (auto& d : swaps) d.solve = 0;
+            for (auto& d : solves) d.swap = 0;
+            mark();
+            launch_panel_rows(ctx, cplx, swaps);
+            mark();
+            launch_panel_rows(ctx, cplx, solves);
+            mark();
+        } else {
+            launch_panel_rows(ctx, cplx, rows);
+        }
         if (!gemms.empty()) gemm_grouped(ctx, gemms, cplx);
         if (timed) mark();
     }
@@ -1764,7 +1756,7 @@ void getrs_free_order(Context& ctx, const DMat& lu, const int* d_piv, DMat& b, i
         const int k0 = kb * bs, w = std::min(bs, n - k0);
         std::vector<TrsmDesc> d{TrsmDesc{lu.p + ((size_t)k0 * ld + k0) * es, ld, b.p + (size_t)k0 * es, ldb, w, nrhs, 1,
                                          adjoint ? 0 : 1, adjoint ? 1 : 0}};
-        launch_trsm(ctx, cplx, 1, d);
+        launch_trsm(ctx, cplx, d);
         update(G + ((size_t)k0 * ldg + k0 + w) * es, b.p + (size_t)k0 * es, b.p + (size_t)(k0 + w) * es, n - k0 - w, w);
     }
     // Backward: U (explicit diagonal) or L^H (unit), then the rows above.
@@ -1772,7 +1764,7 @@ void getrs_free_order(Context& ctx, const DMat& lu, const int* d_piv, DMat& b, i
         const int k0 = kb * bs, w = std::min(bs, n - k0);
         std::vector<TrsmDesc> d{TrsmDesc{lu.p + ((size_t)k0 * ld + k0) * es, ld, b.p + (size_t)k0 * es, ldb, w, nrhs, 0,
                                          adjoint ? 1 : 0, adjoint ? 1 : 0}};
-        launch_trsm(ctx, cplx, 1, d);
+        launch_trsm(ctx, cplx, d);
         update(G + ((size_t)k0 * ldg) * es, b.p + (size_t)k0 * es, b.p, k0, w);
     }
     if (adjoint && d_piv) {
@@ -1912,7 +1904,7 @@ void mixed_trailing(Context& ctx, DMat& a, int j, int w, int moduli) {
     for (int b0 = 0; b0 < w; b0 += 64) {
         const int bw = std::min(64, w - b0);
         std::vector<TrsmDesc> t{TrsmDesc{a.at(j + b0, j + b0), ld, a.at(j + b0, j + w), ld, bw, rest, 1, 1, 0}};
-        launch_trsm(ctx, cplx, 1, t);
+        launch_trsm(ctx, cplx, t);
         if (b0 + bw < w) {
             GemmProblem p{};
             p.A = a.at(j + b0 + bw, j + b0);
@@ -2514,7 +2506,7 @@ void lu_nopiv_panel(Context& ctx, DMat& a, int j, int w, int* flag) {
         }
         if (right > 0) {
             std::vector<TrsmDesc> t{TrsmDesc{a.at(k, k), ld, a.at(k, k + bw), ld, bw, right, 1, 1, 0}};
-            launch_trsm(ctx, cplx, 1, t);
+            launch_trsm(ctx, cplx, t);
             if (below > 0) {
                 GemmProblem p{};
                 p.A = a.at(k + bw, k);

@@ -382,6 +382,10 @@ __global__ void __launch_bounds__(kMaxThreads<CPLX>, 1)
     }
     __syncthreads();
     cluster_sync();  // every CTA's barriers exist before another reaches them
+    // A carried row that moves: its entries, read before any is written.
+    E moved[kW];
+    E* carried = nullptr;
+    int ld = 0, carry = 0;
     if (sl.item >= 0) {
         const PanelFactorDesc& d = batch_item(b, sl.item);
         PanelState<CPLX> s;
@@ -416,10 +420,27 @@ __global__ void __launch_bounds__(kMaxThreads<CPLX>, 1)
         if (ok && s.limit > 8) ok = panel_phase<CPLX, 24>(s, a, pos, 8);
         if (ok && s.limit > 16) ok = panel_phase<CPLX, 16>(s, a, pos, 16);
         if (ok && s.limit > 24) ok = panel_phase<CPLX, 8>(s, a, pos, 24);
-        if (ok && row < M)
+        if (ok && row < M) {
             for (int c = 0; c < d.w; ++c) P[(size_t)c * d.ld + pos] = s.save[(size_t)c * T];
+            if (d.carry > 0 && pos != row) {
+                ld = d.ld;
+                carry = d.carry;
+                const E* from = P - (size_t)carry * ld + row;
+                carried = P - (size_t)carry * ld + pos;
+#pragma unroll
+                for (int c = 0; c < kW; ++c)
+                    if (c < carry) moved[c] = from[(size_t)c * ld];
+            }
+        }
     }
-    cluster_sync();  // nobody leaves while a peer's stores may still be on their way to it
+    // Nobody leaves while a peer's stores may still be on their way to it, and
+    // no carried entry is written before all are read.
+    cluster_sync();
+    if (carried) {
+#pragma unroll
+        for (int c = 0; c < kW; ++c)
+            if (c < carry) carried[(size_t)c * ld] = moved[c];
+    }
 }
 
 // Shared memory of one CTA: the finished entries and both parities' candidate
@@ -490,6 +511,167 @@ void launch(Context& ctx, const std::vector<PanelFactorDesc>& v) {
     ctx.kernel_launches++;
 }
 
+// ---- interchanges and U12 -------------------------------------------------------
+//
+// After a panel, every other column takes the panel's row interchanges and, to
+// the right of it, U12 := L11^-1 A12 (Triangular.SolveLowerUnit,
+// Triangular.cs:26-57; BlockedLu.cs:312-327). One warp per column does both in one
+// pass: every CTA turns the interchanges into moves (which row each touched
+// position ends up with, by following the swaps' references in parallel), the
+// warp loads all of a column's moved rows at once and stores them at their
+// places, and the top w, already in its lanes, go through the triangle first.
+// One thread per column swapping rows in turn took 26 us a step at n = 512, its
+// loads and stores one dependent chain through L2, and the triangle a launch of
+// its own after it.
+
+constexpr int kRowsWarps = 8;
+
+struct PanelMoves {
+    int p[kPanelRowsMaxWidth];      // the swaps' partners
+    int root[kPanelRowsMaxWidth];   // the swap whose own row holds what swap s's own position holds before it
+    int prev[kPanelRowsMaxWidth];   // the latest earlier swap with the same partner, or -1
+    int top[kPanelRowsMaxWidth];    // the row that ends at position k0 + s
+    int dst[kPanelRowsMaxWidth];    // a position beyond the panel's rows that swap s is the last to touch, or -1
+    int src[kPanelRowsMaxWidth];    // and the row that ends there
+};
+
+// Swap s exchanges positions r_s = k0 + s and p_s >= r_s. What r_s holds just
+// before is what the latest earlier swap with partner r_s brought there -- the
+// values its own position held before it, and so on back to a position no swap
+// had touched. Position r_s ends with what p_s holds before swap s; a partner
+// beyond the panel's rows ends with what its last swap's own position held.
+__device__ __forceinline__ void panel_moves(PanelMoves& M, const PanelRowsDesc& d) {
+    const int s = threadIdx.x, w = d.w;
+    if (s < w) M.p[s] = d.swap ? d.piv[d.k0 + s] : d.k0 + s;
+    __syncthreads();
+    int link = -1, prev = -1;
+    bool last = true;
+    const int r = d.k0 + s, p = s < w ? M.p[s] : 0;
+    const bool real = s < w && p != r;
+    if (s < w) {
+        for (int q = 0; q < w; ++q) {
+            const int pq = M.p[q];
+            if (pq == d.k0 + q) continue;  // no swap
+            if (q < s && pq == r) link = q;
+            if (q < s && pq == p) prev = q;
+            if (q > s && pq == p) last = false;
+        }
+        M.root[s] = link < 0 ? s : link;
+        M.prev[s] = prev;
+    }
+    __syncthreads();
+    // Pointer jumping: chains of at most w links.
+    for (int reach = 1; reach < w; reach *= 2) {
+        const int next = s < w ? M.root[M.root[s]] : 0;
+        __syncthreads();
+        if (s < w) M.root[s] = next;
+        __syncthreads();
+    }
+    if (s < w) {
+        const int own = d.k0 + M.root[s];
+        M.top[s] = !real ? own : M.prev[s] >= 0 ? d.k0 + M.root[M.prev[s]] : p;
+        M.dst[s] = real && last && p >= d.k0 + w ? p : -1;
+        M.src[s] = own;
+    }
+    __syncthreads();
+}
+
+template <bool CPLX>
+__global__ void __launch_bounds__(32 * kRowsWarps) panel_rows_kernel(const __grid_constant__ Batch<PanelRowsDesc> b,
+                                                                    int cols_per_cta) {
+    using El_ = El<CPLX>;
+    using E = typename El_::T;
+    int lo = 0, hi = b.count - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (batch_item(b, mid).tile_begin <= (int)blockIdx.x) lo = mid;
+        else hi = mid - 1;
+    }
+    const PanelRowsDesc& d = batch_item(b, lo);
+    extern __shared__ __align__(16) unsigned char panel_smem[];
+    E* t = reinterpret_cast<E*>(panel_smem);  // t[k * w + i] = L11(i, k)
+    __shared__ PanelMoves M;
+    const int w = d.w, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    E* a = reinterpret_cast<E*>(d.a);
+    if (d.solve)
+        for (int e = threadIdx.x; e < w * w; e += 32 * kRowsWarps) {
+            const int k = e / w, i = e - k * w;
+            t[e] = a[(size_t)(d.k0 + k) * d.ld + d.k0 + i];
+        }
+    panel_moves(M, d);  // ends with a block barrier: the triangle is there too
+    const int first = d.c0 + ((int)blockIdx.x - d.tile_begin) * cols_per_cta;
+    for (int c = first + warp; c < min(d.c1, first + cols_per_cta); c += kRowsWarps) {
+        E* col = a + (size_t)c * d.ld;
+        E v[2], out[2];
+        int dst[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int s = lane + 32 * h;
+            dst[h] = -1;
+            v[h] = E{};
+            if (s < w) {
+                v[h] = col[M.top[s]];
+                dst[h] = M.dst[s];
+                if (dst[h] >= 0) out[h] = col[M.src[s]];
+            }
+        }
+        __syncwarp();  // every row is read before one is written
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+            if (dst[h] >= 0) col[dst[h]] = out[h];
+        if (d.solve) {
+            auto pick = [](bool c1, E x, E y) { return c1 ? x : y; };
+            auto bcast = [](E x, int src) {
+                if constexpr (CPLX) return make_double2(__shfl_sync(0xffffffffu, x.x, src), __shfl_sync(0xffffffffu, x.y, src));
+                else return __shfl_sync(0xffffffffu, x, src);
+            };
+#pragma unroll 4
+            for (int k = 0; k < min(w, 32); ++k) {
+                const E x = bcast(v[0], k);
+                const bool nz = El_::nonzero(x);
+                v[0] = pick(nz & (lane > k) & (lane < w), El_::update(v[0], x, t[k * w + min(lane, w - 1)]), v[0]);
+                if (w > 32) v[1] = pick(nz & (lane + 32 < w), El_::update(v[1], x, t[k * w + min(lane + 32, w - 1)]), v[1]);
+            }
+#pragma unroll 4
+            for (int k = 32; k < w; ++k) {
+                const E x = bcast(v[1], k - 32);
+                v[1] = pick(El_::nonzero(x) & (lane + 32 > k) & (lane + 32 < w),
+                            El_::update(v[1], x, t[k * w + min(lane + 32, w - 1)]), v[1]);
+            }
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+            if (lane + 32 * h < w) col[d.k0 + lane + 32 * h] = v[h];
+    }
+}
+
+template <bool CPLX>
+void launch_rows(Context& ctx, std::vector<PanelRowsDesc>& v) {
+    long long cols = 0;
+    int wmax = 0;
+    for (auto& d : v) {
+        cols += d.c1 - d.c0;
+        if (d.solve) wmax = std::max(wmax, d.w);
+    }
+    // A column per warp until the grid is four CTAs per SM; then more.
+    const int per = kRowsWarps * (int)std::max(1LL, cols / (4LL * kRowsWarps * ctx.num_sms));
+    long long total = 0;
+    for (auto& d : v) {
+        d.tile_begin = (int)total;
+        total += (d.c1 - d.c0 + per - 1) / per;
+    }
+    const size_t es = CPLX ? 16 : 8, smem = es * wmax * wmax;
+    static std::atomic<bool> configured[64];
+    if (!configured[ctx.device].load(std::memory_order_acquire)) {
+        TNS_CUDA(cudaFuncSetAttribute(panel_rows_kernel<CPLX>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)(es * kPanelRowsMaxWidth * kPanelRowsMaxWidth)));
+        configured[ctx.device].store(true, std::memory_order_release);
+    }
+    panel_rows_kernel<CPLX><<<(unsigned)total, 32 * kRowsWarps, smem, ctx.stream>>>(make_batch(ctx, v), per);
+    TNS_CUDA(cudaGetLastError());
+    ctx.kernel_launches++;
+}
+
 }  // namespace
 
 int row_panel_max_rows(bool cplx) {
@@ -500,6 +682,15 @@ void launch_row_panels(Context& ctx, bool cplx, const std::vector<PanelFactorDes
     if (v.empty()) return;
     if (cplx) launch<true>(ctx, v);
     else launch<false>(ctx, v);
+}
+
+void launch_panel_rows(Context& ctx, bool cplx, std::vector<PanelRowsDesc>& v) {
+    std::vector<PanelRowsDesc> live;
+    for (auto& d : v)
+        if (d.c1 > d.c0 && d.w > 0 && (d.swap || d.solve)) live.push_back(d);
+    if (live.empty()) return;
+    if (cplx) launch_rows<true>(ctx, live);
+    else launch_rows<false>(ctx, live);
 }
 
 }  // namespace tns
