@@ -12,36 +12,47 @@
 // taylor_kernel. Each matrix is worked on by a group of CTAs ("lanes"); the
 // rows of A, F and the work panels are split among them. One application of
 // A to the n x c work panel X is, per CTA, the product of its rows of A with
-// all of X, staged through shared memory by cp.async in 32-deep k tiles (a
-// 4-stage ring); one thread owns one (row, column) pair and sums in k order
-// with the reference's rounding (PanelProduct.Apply's axpy order, a product
-// and a sum per term; the complex operator's four real sums then
-// (pr - qi, pi + qr), LinearOperators.cs:262-282). The reference skips a term
-// whose x is zero; forming it instead adds +-0 to a sum that is never -0,
-// which changes nothing as long as A is finite, so the skip is kept (as a
-// compare and a select) only in launches with a non-finite operator. The epilogue scales
-// the sums by t/(s(j+1)) into the next work panel, adds them into F and forms
-// both row sums of moduli in column order (InfinityNorm). Every CTA writes
-// its largest row sums to its slot, the group meets at a barrier, and every
-// CTA folds the slots to the same two norms and takes the same exit
-// decision: c1 + c2 <= u ||F||_inf ends the inner loop on the device, with no
-// host round trip. The panels alternate between two buffers, so no CTA
-// overwrites a panel another is still reading.
+// all of X, summed in k order with the reference's rounding (PanelProduct.Apply's
+// axpy order, a product and a sum per term; the complex operator's four real
+// sums then (pr - qi, pi + qr), LinearOperators.cs:262-282). The reference skips
+// a term whose x is zero; forming it instead adds +-0 to a sum that is never
+// -0, which changes nothing as long as A is finite, so the skip is kept (as a
+// compare and a select) only in launches with a non-finite operator. The
+// epilogue scales the sums by t/(s(j+1)) into the next work panel, adds them
+// into F and forms both row sums of moduli in column order (InfinityNorm). The
+// group then meets at a barrier that also exchanges the two norms, and every
+// CTA takes the same exit decision: c1 + c2 <= u ||F||_inf ends the inner loop
+// on the device, with no host round trip. The panels alternate between two
+// buffers, so no CTA overwrites a panel another is still reading.
+//
+// What bounds it: FP64 issue (a product and a sum per term, not fused: 8
+// instructions per complex term, 17.6 cycles of a partition per 4 rows x 8
+// columns) and, per application, the epilogue's and the barrier's latencies.
+// A staging thread keeps a ring of tiles filled by TMA (a box of A, whose
+// first tiles of the next application are fetched while this one ends, and a
+// piece of the row-major X); the multiplying warps hold several rows each,
+// with loads, products and sums of three successive k's in flight. On 24
+// complex matrices (64..1024, 8 columns, 22538 applications) the launch takes
+// 64 ms of which the FP64 instructions alone would take 32; per-thread
+// staging with one row and column per thread, a barrier per tile and a branch
+// per column took 120.
 //
 // Groups and the barrier. A host-side list schedule gives each matrix a width
-// (CTAs) from its share of the batch's work and places it, longest first, on
-// the lanes that free up earliest; each CTA then works through its list of
-// (matrix, rank) in the order of the schedule's start times, which is one
-// total order for every lane, so no group can wait on a lane that waits on
-// it. A group of one CTA synchronises with __syncthreads; a wider group on a
-// counter in global memory (release/acquire), with a bounded spin: a wait
-// gives up after 2 s in which no barrier anywhere in the launch advanced,
-// records a device error and returns, and the host reports TNS_E_TIMEOUT.
+// (CTAs) and places it, longest first, on the lanes that free up earliest;
+// each CTA then works through its list of (matrix, rank) in the order of the
+// schedule's start times, which is one total order for every lane, so no
+// group can wait on a lane that waits on it. A group of one CTA synchronises
+// with __syncthreads; a wider group through slots in global memory, with a
+// bounded spin: a wait gives up after 2 s in which no barrier anywhere in the
+// launch advanced, records a device error and returns, and the host reports
+// TNS_E_TIMEOUT.
 
 #include "batch.cuh"
 #include "device_util.cuh"
 #include "net_compat.h"
 #include "tns_internal.h"
+
+#include <cuda.h>
 
 #include <algorithm>
 #include <cmath>
@@ -49,44 +60,53 @@
 #include <limits>
 #include <numeric>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 namespace tns {
 
 namespace {
 
-constexpr int kThreadsT = 512;  // threads per CTA: (row, column slot) pairs
+constexpr int kMultiplyT = 256;           // threads of the multiplying warps: two groups of four
+constexpr int kThreadsT = kMultiplyT + 32;  // and the staging warp
 
 // The thread layout and the inner loop's form, per launch: SLOTS column slots
-// per row (8 for panels of up to 8 columns, else 16), CPT columns per slot
-// (c + SLOTS q), ROWS = 512 / SLOTS rows per chunk of a CTA's row range.
+// per row, CPT columns per slot (c + SLOTS q), UNIT rows per step of a group
+// of multiplying warps, up to UMAX steps (the first group takes the odd one)
+// and so up to ROWS rows per chunk of a CTA's row range.
 // SKIP keeps the reference's skip of a zero x term explicitly (a compare and
 // a select per term). Without it the term is always formed: that adds +-0 to
 // a sum that is never -0, the same bits whenever A is finite; the host takes
 // that form only when every ||A - mu I||_1 of the launch is finite (0 * inf
 // would otherwise differ from a skip).
-template <int SLOTS_, int CPT_, bool SKIP_>
+template <int SLOTS_, int CPT_, int UMAX_, bool SKIP_>
 struct Shape {
-    static constexpr int SLOTS = SLOTS_, CPT = CPT_, ROWS = kThreadsT / SLOTS_;
+    static constexpr int SLOTS = SLOTS_, CPT = CPT_, UMAX = UMAX_;
+    static constexpr int COLS = SLOTS * CPT, UNIT = 128 / SLOTS, ROWS = UNIT * UMAX;
     static constexpr bool SKIP = SKIP_;
 };
-constexpr int kKT = 32;                    // k per staged tile
-constexpr int kStagesT = 4;                // cp.async ring depth
+// k per staged tile of a chunk's rows and the panel's columns: long tiles where they are few (a
+// tile costs its warps some 200 cycles besides the products). Chunks stop at
+// 112 rows, of which three stages of 32 fit; 128 rows in stages of 16 took
+// 207 to 222 cycles a k, 112 rows 150 (8 columns, complex).
+__host__ __device__ constexpr int tile_k(int rows, int cols) {
+    return rows + cols <= 24 ? 128 : rows + cols <= 40 ? 64 : 32;
+}
+constexpr int kStagesMax = 8;              // ring depth, as far as kSmemT holds it
+constexpr size_t kSmemT = 222 * 1024;      // dynamic shared memory of a CTA
 constexpr double kU = 1.1102230246251565e-16;
 constexpr int kDevTimeoutGroup = 4;  // DeviceError: a group barrier of the Taylor kernel gave up
 
 struct TaylorDesc {
-    const double* a;   // the shifted matrix A - mu I, ld lda
     const double* b;   // B, ld ldb
     double* f;         // the result F, ld ldp
-    double* w0;        // work panels, ld ldp
+    double* w0;        // work panels, row-major, COLS wide
     double* w1;
     const double* coeff;        // m coefficients t / (s (j + 1))
-    double* partials;           // [2][width][2]
-    unsigned long long* bar;    // the group's barrier counter (zero at launch)
+    unsigned long long* slots;  // [3][width][2] norms, kEmpty until published
     int* out;                   // [applications, early exits]
-    int n, lda, ldb, ldp;
-    int m, s, width, rows_per;  // rows_per: rows per CTA, a multiple of 8
+    int n, ldb, ldp;
+    int m, s, width, chunk, rows_per;  // rows_per: rows per CTA and per chunk of them, multiples of the launch's UNIT
     double eta_re, eta_im;
     int eta_one;
 };
@@ -98,153 +118,137 @@ struct TaylorPlan {
 struct TaylorLaunch {
     const TaylorDesc* descs;
     const TaylorPlan* plan;
+    const CUtensorMap* maps;  // of each shifted matrix, boxes of a chunk's rows by tile_k columns
     const int* plan_off;  // gridDim.x + 1 offsets into plan
     int ncols;
     int* err;
     unsigned long long* progress;  // every barrier arrival in the launch
 };
 
-__device__ __forceinline__ void cp16(void* dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
+// Orders this thread's plain accesses to global memory with bulk copies of it.
+__device__ __forceinline__ void fence_async_global() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
+__device__ __forceinline__ void mbar_inval(uint64_t* bar) {
+    asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(smem_addr(bar)) : "memory");
 }
-__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_wait() {
-    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-__device__ __forceinline__ unsigned long long ld_acquire(const unsigned long long* p) {
+__device__ __forceinline__ unsigned long long ld_relaxed(const unsigned long long* p) {
     unsigned long long v;
-    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
     return v;
 }
-
-// The group's barrier number `target / width`. False when it gave up (the
-// error flag is then set); every thread of the CTA gets the same answer.
-__device__ bool group_sync(const TaylorDesc& d, unsigned long long target, const TaylorLaunch& L, int* s_flag) {
-    __syncthreads();
-    if (d.width == 1) return true;
-    if (threadIdx.x == 0) {
-        __threadfence();
-        atomicAdd(d.bar, 1ull);
-        atomicAdd(L.progress, 1ull);
-        int ok = 1;
-        if (ld_acquire(d.bar) < target) {
-            unsigned long long start = global_timer_ns();
-            unsigned long long beat = ld_acquire(L.progress);
-            for (unsigned it = 1;; ++it) {
-                if (ld_acquire(d.bar) >= target) break;
-                if (it > 64) __nanosleep(64);
-                if ((it & 127u) == 0) {
-                    if (*reinterpret_cast<volatile int*>(L.err) != 0) {
-                        ok = 0;
-                        break;
-                    }
-                    const unsigned long long now = global_timer_ns();
-                    const unsigned long long b2 = ld_acquire(L.progress);
-                    if (b2 != beat) {
-                        beat = b2;
-                        start = now;
-                    } else if (now - start > kWaitTimeoutNs) {
-                        atomicCAS(L.err, 0, kDevTimeoutGroup);
-                        ok = 0;
-                        break;
-                    }
-                }
-            }
-        }
-        __threadfence();
-        *s_flag = ok;
-    }
-    __syncthreads();
-    return *s_flag != 0;
+// Two words, each read whole.
+__device__ __forceinline__ ulonglong2 ld_acquire2(const unsigned long long* p) {
+    ulonglong2 v;
+    asm volatile("ld.acquire.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_relaxed(unsigned long long* p, unsigned long long v) {
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
-// Largest of non-negative values with Math.Max's NaN rule (any NaN wins).
+// Largest of non-negative values with Math.Max's NaN rule (any NaN wins):
+// their bits order as the values do, a quiet NaN above infinity.
 struct NormAcc {
-    double v = 0.0;
-    bool nan = false;
-    __device__ void add(double x) {
-        if (isnan(x)) nan = true;
-        else if (x > v) v = x;
+    unsigned long long bits = 0;
+    __device__ void add(double x) { join(isnan(x) ? 0x7ff8000000000000ull : (unsigned long long)__double_as_longlong(x)); }
+    __device__ void join(unsigned long long b) { bits = b > bits ? b : bits; }
+    // Over the warp: the high words' largest, then the low words' among its.
+    __device__ void fold() {
+        const unsigned hi = (unsigned)(bits >> 32), top = __reduce_max_sync(0xffffffffu, hi);
+        const unsigned lo = hi == top ? (unsigned)bits : 0u;
+        bits = ((unsigned long long)top << 32) | __reduce_max_sync(0xffffffffu, lo);
     }
-    __device__ double value() const { return nan ? __longlong_as_double(0x7ff8000000000000ll) : v; }
+};
+constexpr unsigned long long kEmpty = ~0ull;  // a slot not yet published (no norm has these bits)
+
+struct NormShared {
+    unsigned long long warp[2][kThreadsT / 32];
+    double norm[2];
+    int ok;
 };
 
-// Fold the CTA's two norm accumulators (every thread holds its own) into
-// s_part[0..1] (thread 0's view after the sync).
-__device__ void cta_fold(NormAcc a0, NormAcc a1, double* s_red, int* s_nan, double* s_part) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        double x0 = __shfl_xor_sync(0xffffffffu, a0.v, o), x1 = __shfl_xor_sync(0xffffffffu, a1.v, o);
-        int n0 = __shfl_xor_sync(0xffffffffu, (int)a0.nan, o), n1 = __shfl_xor_sync(0xffffffffu, (int)a1.nan, o);
-        a0.v = x0 > a0.v ? x0 : a0.v;
-        a1.v = x1 > a1.v ? x1 : a1.v;
-        a0.nan = a0.nan || n0;
-        a1.nan = a1.nan || n1;
-    }
-    if (lane == 0) {
-        s_red[warp] = a0.v;
-        s_red[32 + warp] = a1.v;
-        s_nan[warp] = a0.nan;
-        s_nan[32 + warp] = a1.nan;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        NormAcc r0, r1;
-        for (int w = 0; w < kThreadsT / 32; ++w) {
-            r0.v = s_red[w] > r0.v ? s_red[w] : r0.v;
-            r1.v = s_red[32 + w] > r1.v ? s_red[32 + w] : r1.v;
-            r0.nan = r0.nan || s_nan[w];
-            r1.nan = r1.nan || s_nan[32 + w];
+// Join the group's published words of this lane's ranks, all of them asked
+// for at once until each is there. False when the wait gave up.
+__device__ bool await_slots(const unsigned long long* slots, int width, const TaylorLaunch& L, NormAcc& r0, NormAcc& r1) {
+    unsigned long long start = 0, beat = 0;
+    for (unsigned it = 0;; ++it) {
+        bool all = true;
+        for (int r = threadIdx.x; r < width; r += 32) {
+            const ulonglong2 v = ld_acquire2(slots + 2 * r);
+            if (v.x != kEmpty) r0.join(v.x);
+            if (v.y != kEmpty) r1.join(v.y);
+            all = all && v.x != kEmpty && v.y != kEmpty;
         }
-        s_part[0] = r0.value();
-        s_part[1] = r1.value();
+        if (all) return true;
+        if (it > 64) __nanosleep(64);
+        if ((it & 127u) == 0) {
+            if (*reinterpret_cast<volatile int*>(L.err) != 0) return false;
+            const unsigned long long now = global_timer_ns(), b2 = ld_relaxed(L.progress);
+            if (it == 0 || b2 != beat) {
+                beat = b2;
+                start = now;
+            } else if (now - start > kWaitTimeoutNs) {
+                atomicCAS(L.err, 0, kDevTimeoutGroup);
+                return false;
+            }
+        }
     }
 }
 
-// Publish the CTA's two values, meet the group, and leave the group's two
-// norms in s_norm (every thread). False if the barrier gave up.
-__device__ bool group_norms(const TaylorDesc& d, int rank, unsigned long long& phase, const TaylorLaunch& L,
-                            NormAcc a0, NormAcc a1, double* s_red, int* s_nan, double* s_part, double* s_norm,
-                            int* s_flag) {
-    cta_fold(a0, a1, s_red, s_nan, s_part);
-    const int parity = (int)(phase & 1);
-    if (d.width > 1 && threadIdx.x == 0) {
-        double* slot = d.partials + ((size_t)parity * d.width + rank) * 2;
-        slot[0] = s_part[0];
-        slot[1] = s_part[1];
-    }
-    ++phase;
-    if (!group_sync(d, phase * (unsigned long long)d.width, L, s_flag)) return false;
-    if (d.width == 1) {
-        if (threadIdx.x == 0) {
-            s_norm[0] = s_part[0];
-            s_norm[1] = s_part[1];
-        }
-    } else if (threadIdx.x < 32) {
-        NormAcc r0, r1;
-        for (int r = threadIdx.x; r < d.width; r += 32) {
-            const double* slot = d.partials + ((size_t)parity * d.width + r) * 2;
-            r0.add(__ldcg(slot));
-            r1.add(__ldcg(slot + 1));
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            double x0 = __shfl_xor_sync(0xffffffffu, r0.v, o), x1 = __shfl_xor_sync(0xffffffffu, r1.v, o);
-            int n0 = __shfl_xor_sync(0xffffffffu, (int)r0.nan, o), n1 = __shfl_xor_sync(0xffffffffu, (int)r1.nan, o);
-            r0.v = x0 > r0.v ? x0 : r0.v;
-            r1.v = x1 > r1.v ? x1 : r1.v;
-            r0.nan = r0.nan || n0;
-            r1.nan = r1.nan || n1;
-        }
-        if (threadIdx.x == 0) {
-            s_norm[0] = r0.value();
-            s_norm[1] = r1.value();
-        }
+// The group's barrier and its two norms (sh.norm, every thread): each CTA
+// publishes its own two and reads everyone's, so that arriving and giving the
+// value are one store, and waiting and reading it one load (4600 cycles for a
+// group of 4 with a counter, a fence on each side and the values read after
+// it; 2700 to 3500 so).
+// Slots rotate over three phases. A CTA empties its slot of phase p + 2 after
+// it has seen all of phase p, when everyone has read phase p - 1, the slot's
+// last use; and it publishes p + 1, which everyone awaits before p + 2, after
+// that. False if a wait gave up here or on the ring of tiles.
+__device__ bool group_norms(const TaylorDesc& d, int rank, unsigned& phase, const TaylorLaunch& L, NormAcc a0,
+                            NormAcc a1, NormShared& sh, const int* s_dead) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    fence_async_global();  // this thread's part of the work panel, before the group's copies of it
+    a0.fold();
+    a1.fold();
+    if (lane == 0) {
+        sh.warp[0][warp] = a0.bits;
+        sh.warp[1][warp] = a1.bits;
     }
     __syncthreads();
-    return true;
+    if (warp == 0) {
+        NormAcc r0, r1;
+        if (lane < kThreadsT / 32) {
+            r0.bits = sh.warp[0][lane];
+            r1.bits = sh.warp[1][lane];
+        }
+        r0.fold();
+        r1.fold();
+        bool ok = true;
+        if (d.width > 1) {
+            unsigned long long* slots = d.slots + (size_t)phase * d.width * 2;
+            if (lane == 0) {
+                asm volatile("fence.acq_rel.gpu;" ::: "memory");
+                st_relaxed(slots + 2 * rank, r0.bits);
+                st_relaxed(slots + 2 * rank + 1, r1.bits);
+            }
+            ok = await_slots(slots, d.width, L, r0, r1);
+            __syncwarp();
+            r0.fold();
+            r1.fold();
+            ok = __all_sync(0xffffffffu, ok);
+            phase = phase == 2 ? 0 : phase + 1;
+            if (lane == 0) atomicAdd(L.progress, 1ull);  // the launch is alive
+            if (lane < 2) st_relaxed(d.slots + (size_t)(phase == 2 ? 0 : phase + 1) * d.width * 2 + 2 * rank + lane, kEmpty);
+        }
+        if (lane == 0) {
+            sh.norm[0] = __longlong_as_double((long long)r0.bits);
+            sh.norm[1] = __longlong_as_double((long long)r1.bits);
+            sh.ok = ok;
+        }
+    } else if (d.width > 1) {
+        phase = phase == 2 ? 0 : phase + 1;
+    }
+    __syncthreads();
+    return sh.ok && !*s_dead;
 }
 
 template <bool CPLX>
@@ -272,143 +276,287 @@ __device__ __forceinline__ double row_sum(const double (&v)[S::CPT], int ncols) 
 
 template <bool CPLX, class S>
 struct Tiles {
-    static constexpr int ES = CPLX ? 2 : 1;                 // doubles per element
-    static constexpr int XS = CPLX ? kKT + 1 : kKT + 2;     // elements per staged X column
-    static constexpr int A_DOUBLES = kKT * S::ROWS * ES;
-    static constexpr int X_DOUBLES = S::SLOTS * S::CPT * XS * ES;
-    static constexpr int STAGE = A_DOUBLES + X_DOUBLES;
-    static constexpr size_t SMEM = sizeof(double) * (size_t)STAGE * kStagesT;
+    static constexpr int ES = CPLX ? 2 : 1;              // doubles per element
+    static constexpr int Y_DOUBLES = S::ROWS * S::COLS * ES;  // of the products, and of F
+    // One stage for chunks of up to `units` steps of rows, and how many fit.
+    static __host__ __device__ constexpr int stage_doubles(int units) {
+        return tile_k(S::UNIT * units, S::COLS) * (S::UNIT * units + S::COLS) * ES;
+    }
+    static __device__ __forceinline__ int stages(int units) {
+        return min(kStagesMax, (int)((kSmemT / sizeof(double) - 2 * Y_DOUBLES) / stage_doubles(units)));
+    }
+    static_assert(stage_doubles(S::UMAX) * 3 + 2 * Y_DOUBLES <= (int)(kSmemT / sizeof(double)), "three stages");
+    static_assert(S::ROWS * ES <= 256, "the rows of a tensor-map box");
+    static_assert(S::UNIT * S::COLS * ES * 8 % 128 == 0, "TMA destinations at multiples of 128 bytes");
 };
 
-// Stage k tile [k0, k0 + kKT) of the CTA's rows [r0, r0 + rows) of A and of
-// the work panel x (all columns) into stage buffer `buf`.
-template <bool CPLX, class S>
-__device__ __forceinline__ void stage_tile(double* buf, const TaylorDesc& d, const double* x, int ncols, int r0,
-                                           int rows, int k0) {
-    using T = Tiles<CPLX, S>;
-    constexpr int R = S::ROWS;
-    double* sA = buf;
-    double* sX = buf + T::A_DOUBLES;
-    const int tid = threadIdx.x;
-    if constexpr (CPLX) {
-        for (int e = tid; e < kKT * R; e += kThreadsT) {
-            const int k = e / R, r = e % R;
-            if (r < rows) cp16(sA + (k * R + r) * 2, d.a + ((size_t)(k0 + k) * d.lda + r0 + r) * 2);
-        }
-        for (int e = tid; e < ncols * kKT; e += kThreadsT) {
-            const int col = e / kKT, k = e % kKT;
-            cp16(sX + (col * T::XS + k) * 2, x + ((size_t)col * d.ldp + k0 + k) * 2);
-        }
-    } else {
-        for (int e = tid; e < kKT * (R / 2); e += kThreadsT) {
-            const int k = e / (R / 2), rp = (e % (R / 2)) * 2;
-            if (rp < rows) cp16(sA + k * R + rp, d.a + (size_t)(k0 + k) * d.lda + r0 + rp);
-        }
-        for (int e = tid; e < ncols * (kKT / 2); e += kThreadsT) {
-            const int col = e / (kKT / 2), kp = (e % (kKT / 2)) * 2;
-            cp16(sX + col * T::XS + kp, x + (size_t)col * d.ldp + k0 + kp);
+// A position in the ring of staged tiles: the slot and the parity of its lap.
+struct Ring {
+    int slot = 0;
+    unsigned lap = 0;
+    __device__ void next(int stages) {
+        if (++slot == stages) {
+            slot = 0;
+            lap ^= 1;
         }
     }
-}
+};
 
-// acc := (rows r0.. of A) * x for this thread's (row, columns), in k order.
+struct RingBars {
+    uint64_t full[kStagesMax], empty[kStagesMax];
+    int dead;  // a wait on the ring gave up
+};
+
+// The staging warp's side, one thread of it: k tile [k0, k0 + kt) of the
+// CTA's rows r0... of A into a slot of the ring, one box of `units` steps of
+// rows (those past the matrix come as zeros), and the same rows of the work
+// panel. (Copies of single columns of the tile kept the staging warp busy for
+// 1900 cycles a tile, and per-thread copies four warps for 2900, against 900
+// to multiply 16 rows of it.)
 template <bool CPLX, class S>
-__device__ __forceinline__ void product_chunk(double* smem, const TaylorDesc& d, const double* x, int ncols, int r0,
-                                              int rows, double (&acc)[S::CPT][CPLX ? 4 : 1]) {
+struct Stager {
     using T = Tiles<CPLX, S>;
-    constexpr int R = S::ROWS;
-    const int rr = threadIdx.x / S::SLOTS, c = threadIdx.x % S::SLOTS;
-#pragma unroll
-    for (int q = 0; q < S::CPT; ++q)
-#pragma unroll
-        for (int z = 0; z < (CPLX ? 4 : 1); ++z) acc[q][z] = 0.0;
-    const int n = d.n;
-    const int ktiles = (n + kKT - 1) / kKT;
-#pragma unroll
-    for (int st = 0; st < kStagesT - 1; ++st) {
-        if (st < ktiles) stage_tile<CPLX, S>(smem + st * T::STAGE, d, x, ncols, r0, rows, st * kKT);
-        cp_commit();
+    const TaylorDesc& d;
+    const CUtensorMap* map;
+    double* smem;
+    RingBars& bars;
+    int* err;
+    int units, kt, stages, stage_doubles;
+    Ring a, x;  // the next tile of A and of X
+
+    __device__ __forceinline__ bool put_a(int r0, int k0) {
+        if (!mbar_wait_bounded(&bars.empty[a.slot], a.lap ^ 1, err, kDevTimeoutEmpty)) {
+            bars.dead = 1;
+            return false;
+        }
+        mbar_arrive_expect_tx(&bars.full[a.slot], kt * S::UNIT * units * T::ES * 8);
+        tma_load_2d(smem + (size_t)a.slot * stage_doubles, map, r0 * T::ES, k0, &bars.full[a.slot]);
+        a.next(stages);
+        return true;
     }
-    bool col_ok[S::CPT];
+    __device__ __forceinline__ void put_x(const double* w, int k0) {
+        const uint32_t bytes = min(kt, d.n - k0) * S::COLS * T::ES * 8;
+        mbar_arrive_expect_tx(&bars.full[x.slot], bytes);
+        bulk_copy_g2s(smem + (size_t)x.slot * stage_doubles + kt * S::UNIT * units * T::ES,
+                      w + (size_t)k0 * S::COLS * T::ES, bytes, &bars.full[x.slot]);
+        x.next(stages);
+    }
+    // Tiles of A without their X: take their copies in, so that none is under
+    // way when the slots are given up; likewise, after a wait that gave up,
+    // the last tile of every slot.
+    __device__ void drain() {
+        while (x.slot != a.slot || x.lap != a.lap) {
+            mbar_arrive(&bars.full[x.slot]);
+            x.next(stages);
+        }
+        for (int s = 0; s < stages; ++s)
+            mbar_wait_bounded(&bars.full[s], s < a.slot ? a.lap : a.lap ^ 1, err, kDevTimeoutDrain);
+    }
+};
+
+// Steps of rows of the first group of four multiplying warps: all of up to
+// three, half from four on. One warp per partition with two rows a thread
+// takes 41 cycles a k, two with one each 54; with four and two 76 and 75, and
+// beyond that two warps hide each other's latencies (8 columns, complex).
+__host__ __device__ constexpr int first_steps(int units) { return units <= 3 ? units : (units + 1) / 2; }
+
+// The multiplying warps' side: Y := (rows of the chunk of A) X over all k
+// tiles, in k order, into sY (row-major, COLS wide). Thread (row, column) of
+// a group holds rows row + UNIT (base + q): a warp reads RT + CPT operands
+// for 8 RT CPT (complex) FP64 instructions. The operands of k + 2 are loaded
+// and the products of k + 1 formed while those of k are added, across the
+// tiles' ends. Columns past ncols repeat the last.
+template <bool CPLX, class S, int RT>
+__device__ __forceinline__ void multiply_chunk(double* smem, RingBars& bars, Ring& ring, int stages, int stage_doubles,
+                                               int kt, int pitch, int base, int n, int ncols, double* sY, int* err) {
+    using T = Tiles<CPLX, S>;
+    constexpr int CPT = S::CPT;
+    using Elem = std::conditional_t<CPLX, double2, double>;
+    // Bit 1 of the lane counts rows and bit 0 columns, so that lanes a bit
+    // apart read the same operand: a 16-byte read of a warp then takes two
+    // passes instead of four, of A and of X both.
+    const int lane = threadIdx.x & 31, c = (lane & 1) | ((lane >> 1) & (S::SLOTS - 2));
+    const int rr = base * S::UNIT + (threadIdx.x % 128 >> 5) * (32 / S::SLOTS) +
+                   (((lane >> 1) & 1) | (lane / (2 * S::SLOTS) * 2));
+    double acc[RT][CPT][CPLX ? 4 : 1];
 #pragma unroll
-    for (int q = 0; q < S::CPT; ++q) col_ok[q] = c + q * S::SLOTS < ncols;
-    for (int kt = 0; kt < ktiles; ++kt) {
-        cp_wait<kStagesT - 2>();
-        __syncthreads();
-        const int nxt = kt + kStagesT - 1;
-        if (nxt < ktiles) stage_tile<CPLX, S>(smem + (nxt % kStagesT) * T::STAGE, d, x, ncols, r0, rows, nxt * kKT);
-        cp_commit();
-        const double* sA = smem + (kt % kStagesT) * T::STAGE;
-        const double* sX = sA + T::A_DOUBLES;
-        const int klen = min(kKT, n - kt * kKT);
-        if (rr < rows) {
-            if constexpr (CPLX) {
-                const double2* a2 = reinterpret_cast<const double2*>(sA) + rr;
-                const double2* x2 = reinterpret_cast<const double2*>(sX) + c * T::XS;
-#pragma unroll 4
-                for (int kk = 0; kk < klen; ++kk) {
-                    const double2 av = a2[kk * R];
+    for (int q = 0; q < RT; ++q)
 #pragma unroll
-                    for (int q = 0; q < S::CPT; ++q) {
-                        if (!col_ok[q]) continue;
-                        const double2 xv = x2[q * S::SLOTS * T::XS + kk];
-                        if constexpr (S::SKIP) {
-                            const bool nr = xv.x != 0.0, ni = xv.y != 0.0;
-                            acc[q][0] = add_rn(acc[q][0], nr ? mul_rn(xv.x, av.x) : 0.0);  // pr
-                            acc[q][2] = add_rn(acc[q][2], nr ? mul_rn(xv.x, av.y) : 0.0);  // qr
-                            acc[q][1] = add_rn(acc[q][1], ni ? mul_rn(xv.y, av.x) : 0.0);  // pi
-                            acc[q][3] = add_rn(acc[q][3], ni ? mul_rn(xv.y, av.y) : 0.0);  // qi
-                        } else {
-                            acc[q][0] = add_rn(acc[q][0], mul_rn(xv.x, av.x));
-                            acc[q][2] = add_rn(acc[q][2], mul_rn(xv.x, av.y));
-                            acc[q][1] = add_rn(acc[q][1], mul_rn(xv.y, av.x));
-                            acc[q][3] = add_rn(acc[q][3], mul_rn(xv.y, av.y));
-                        }
-                    }
-                }
-            } else {
-                const double* a1 = sA + rr;
-                const double* x1 = sX + c * T::XS;
-#pragma unroll 4
-                for (int kk = 0; kk < klen; ++kk) {
-                    const double av = a1[kk * R];
+        for (int p = 0; p < CPT; ++p)
 #pragma unroll
-                    for (int q = 0; q < S::CPT; ++q) {
-                        if (!col_ok[q]) continue;
-                        const double xv = x1[q * S::SLOTS * T::XS + kk];
-                        if constexpr (S::SKIP) acc[q][0] = add_rn(acc[q][0], xv != 0.0 ? mul_rn(xv, av) : 0.0);
-                        else acc[q][0] = add_rn(acc[q][0], mul_rn(xv, av));
-                    }
+            for (int z = 0; z < (CPLX ? 4 : 1); ++z) acc[q][p][z] = 0.0;
+    int xoff[CPT];
+#pragma unroll
+    for (int p = 0; p < CPT; ++p) xoff[p] = min(c + p * S::SLOTS, ncols - 1);
+    bool alive = true;
+    const Elem *sA, *sX;
+    Elem av[2][RT], xv[2][CPT];
+    // The next tile. After a wait that gave up the sums are of no use, and the
+    // CTA returns at its next barrier.
+    auto take = [&] {
+        if (alive && !mbar_wait_bounded(&bars.full[ring.slot], ring.lap, err, kDevTimeoutFull)) {
+            alive = false;
+            bars.dead = 1;
+        }
+        sA = reinterpret_cast<const Elem*>(smem + (size_t)ring.slot * stage_doubles) + rr;
+        sX = reinterpret_cast<const Elem*>(smem + (size_t)ring.slot * stage_doubles) + kt * pitch;
+    };
+    auto load = [&](int b, int k) {
+#pragma unroll
+        for (int q = 0; q < RT; ++q) av[b][q] = sA[k * pitch + q * S::UNIT];
+#pragma unroll
+        for (int p = 0; p < CPT; ++p) xv[b][p] = sX[k * S::COLS + xoff[p]];
+    };
+    double pr[2][RT][CPT][CPLX ? 4 : 1];
+    auto multiply = [&](int b) {
+#pragma unroll
+        for (int q = 0; q < RT; ++q)
+#pragma unroll
+            for (int p = 0; p < CPT; ++p) {
+                if constexpr (CPLX) {
+                    const double2 a = av[b][q], x = xv[b][p];
+                    const bool nr = !S::SKIP || x.x != 0.0, ni = !S::SKIP || x.y != 0.0;
+                    pr[b][q][p][0] = nr ? mul_rn(x.x, a.x) : 0.0;  // pr
+                    pr[b][q][p][1] = ni ? mul_rn(x.y, a.x) : 0.0;  // pi
+                    pr[b][q][p][2] = nr ? mul_rn(x.x, a.y) : 0.0;  // qr
+                    pr[b][q][p][3] = ni ? mul_rn(x.y, a.y) : 0.0;  // qi
+                } else {
+                    const double a = av[b][q], x = xv[b][p];
+                    pr[b][q][p][0] = !S::SKIP || x != 0.0 ? mul_rn(x, a) : 0.0;
                 }
             }
+    };
+    auto add = [&](int b) {
+#pragma unroll
+        for (int q = 0; q < RT; ++q)
+#pragma unroll
+            for (int p = 0; p < CPT; ++p)
+#pragma unroll
+                for (int z = 0; z < (CPLX ? 4 : 1); ++z) acc[q][p][z] = add_rn(acc[q][p][z], pr[b][q][p][z]);
+    };
+    take();
+    load(0, 0);
+    load(1, 1);
+    multiply(0);
+    for (int k0 = 0; k0 < n; k0 += kt) {
+        const int klen = min(kt, n - k0);
+        const bool more = k0 + kt < n;
+        uint64_t* done = &bars.empty[ring.slot];
+        ring.next(stages);
+        // (loads past the last k: whatever the slot holds there, not used)
+        int kk = 0;
+        for (; kk + 4 <= klen - (more ? 4 : 0); kk += 4) {
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                load(u & 1, kk + u + 2);
+                multiply((u + 1) & 1);
+                add(u & 1);
+            }
         }
+        if (more) {
+            // The last four, with the first operands of the next tile.
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                if (u == 2) take();
+                load(u & 1, u < 2 ? kk + u + 2 : u - 2);
+                multiply((u + 1) & 1);
+                add(u & 1);
+            }
+        } else {
+#pragma unroll
+            for (int u = 0; u < 3; ++u)
+                if (kk + u < klen) {
+                    load(u & 1, kk + u + 2);
+                    multiply((u + 1) & 1);
+                    add(u & 1);
+                }
+        }
+        __syncwarp();
+        if ((threadIdx.x & 31) == 0) mbar_arrive(done);
     }
-    cp_wait<0>();
-    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < RT; ++q)
+#pragma unroll
+        for (int p = 0; p < CPT; ++p) {
+            double* y = sY + ((q * S::UNIT + rr) * S::COLS + c + p * S::SLOTS) * T::ES;
+            if constexpr (CPLX) {
+                // the reference's four real sums combine as (pr - qi, pi + qr)
+                *reinterpret_cast<double2*>(y) = make_double2(sub_rn(acc[q][p][0], acc[q][p][3]), add_rn(acc[q][p][1], acc[q][p][2]));
+            } else {
+                y[0] = acc[q][p][0];
+            }
+        }
+}
+
+template <bool CPLX, class S, int RT = (S::UMAX > 6 ? (S::UMAX + 1) / 2 : 3)>
+__device__ __forceinline__ void multiply_dispatch(int rt, double* smem, RingBars& bars, Ring& ring, int stages,
+                                                  int stage_doubles, int kt, int pitch, int base, int n, int ncols, double* sY,
+                                                  int* err) {
+    if constexpr (RT == 0) {
+        // The second group of a chunk of one step: frees the tiles unread.
+        for (int k0 = 0; k0 < n; k0 += kt) {
+            if (!mbar_wait_bounded(&bars.full[ring.slot], ring.lap, err, kDevTimeoutFull)) bars.dead = 1;
+            __syncwarp();
+            if ((threadIdx.x & 31) == 0) mbar_arrive(&bars.empty[ring.slot]);
+            ring.next(stages);
+        }
+    } else {
+        if (rt == RT)
+            return multiply_chunk<CPLX, S, RT>(smem, bars, ring, stages, stage_doubles, kt, pitch, base, n, ncols, sY, err);
+        multiply_dispatch<CPLX, S, RT - 1>(rt, smem, bars, ring, stages, stage_doubles, kt, pitch, base, n, ncols, sY, err);
+    }
 }
 
 template <bool CPLX, class S>
 __global__ void __launch_bounds__(kThreadsT, 1) taylor_kernel(const __grid_constant__ TaylorLaunch L) {
-    constexpr int CPT = S::CPT, R = S::ROWS;
+    using T = Tiles<CPLX, S>;
+    constexpr int CPT = S::CPT, ES = T::ES;
+    constexpr int RP = kMultiplyT / S::SLOTS;  // rows of one pass of the element-wise parts
     extern __shared__ __align__(128) double smem[];
-    __shared__ double s_red[64];
-    __shared__ int s_nan[64];
-    __shared__ double s_part[2];
-    __shared__ double s_norm[2];
-    __shared__ int s_flag;
+    __shared__ RingBars bars;
+    __shared__ NormShared sh;
+    double* const sY = smem + kSmemT / sizeof(double) - 2 * T::Y_DOUBLES;
+    double* const sF = sY + T::Y_DOUBLES;
     const int ncols = L.ncols;
-    const int rr = threadIdx.x / S::SLOTS, cs = threadIdx.x % S::SLOTS;
+    const bool multiplying = threadIdx.x < kMultiplyT;
+    const int rr = multiplying ? threadIdx.x / S::SLOTS : 1 << 28, cs = threadIdx.x % S::SLOTS;
+    const bool staging = threadIdx.x == kMultiplyT;
+    if (threadIdx.x == 0) bars.dead = 0;
     for (int e = L.plan_off[blockIdx.x]; e < L.plan_off[blockIdx.x + 1]; ++e) {
         const TaylorPlan pl = L.plan[e];
         const TaylorDesc d = L.descs[pl.matrix];
         const int rank = pl.rank;
         const int rbeg = rank * d.rows_per, rend = min(d.n, rbeg + d.rows_per);
-        unsigned long long phase = 0;
-        const size_t es = CPLX ? 2 : 1;
+        const int R = d.chunk, units = R / S::UNIT, kt = tile_k(R, S::COLS);  // of the staged boxes
+        const int ktiles = (d.n + kt - 1) / kt;
+        const int stage_doubles = T::stage_doubles(units), stages = T::stages(units);
+        unsigned phase = 0;
+        if (threadIdx.x == 0) {
+            for (int i = 0; i < stages; ++i) {
+                mbar_init(&bars.full[i], 2);
+                mbar_init(&bars.empty[i], kMultiplyT / 32);
+            }
+            mbar_fence_init();
+        }
+        __syncthreads();
+        // A does not change: its first tiles of the next product are copied
+        // ahead of the barrier that X waits for.
+        Ring ring;  // the multiplying warps' next tile
+        Stager<CPLX, S> st{d, L.maps + pl.matrix, smem, bars, L.err, units, kt, stages, stage_doubles};
+        const int ahead = min(stages, ktiles);
+        // F stays in shared memory to the end where the CTA's rows are one chunk.
+        const bool f_local = rend - rbeg <= R;
+        auto f_at = [&](int i, int col) {
+            return f_local ? sF + ((i - rbeg) * S::COLS + col) * ES : d.f + ((size_t)col * d.ldp + i) * ES;
+        };
+        if (staging) {
+            tensormap_acquire(st.map);
+            for (int t = 0; t < ahead && st.put_a(rbeg, t * kt); ++t) {}
+        }
 
         // F := B, work := B, c1 = ||B||_inf (Run, :274-276, :285).
         NormAcc n0, n1;
-        for (int r0 = rbeg; r0 < rend; r0 += R) {
+        for (int r0 = rbeg; r0 < rend; r0 += RP) {
             const int i = r0 + rr;
             const bool row_ok = i < rend;
             double v[CPT];
@@ -417,13 +565,15 @@ __global__ void __launch_bounds__(kThreadsT, 1) taylor_kernel(const __grid_const
                 const int col = cs + q * S::SLOTS;
                 v[q] = 0.0;
                 if (row_ok && col < ncols) {
-                    const size_t bi = ((size_t)col * d.ldb + i) * es, pi = ((size_t)col * d.ldp + i) * es;
+                    const size_t bi = ((size_t)col * d.ldb + i) * ES;
+                    double* f = f_at(i, col);
+                    const size_t wi = ((size_t)i * S::COLS + col) * ES;
                     const double re = d.b[bi], im = CPLX ? d.b[bi + 1] : 0.0;
-                    d.f[pi] = re;
-                    d.w0[pi] = re;
+                    f[0] = re;
+                    d.w0[wi] = re;
                     if (CPLX) {
-                        d.f[pi + 1] = im;
-                        d.w0[pi + 1] = im;
+                        f[1] = im;
+                        d.w0[wi + 1] = im;
                     }
                     v[q] = modulus<CPLX>(re, im);
                 }
@@ -431,8 +581,11 @@ __global__ void __launch_bounds__(kThreadsT, 1) taylor_kernel(const __grid_const
             const double rs = row_sum<S>(v, ncols);
             if (row_ok) n0.add(rs);
         }
-        if (!group_norms(d, rank, phase, L, n0, n1, s_red, s_nan, s_part, s_norm, &s_flag)) return;
-        double c1 = s_norm[0];
+        if (!group_norms(d, rank, phase, L, n0, n1, sh, &bars.dead)) {
+            if (staging) st.drain();
+            return;
+        }
+        double c1 = sh.norm[0];
 
         int applications = 0, early = 0;
         double* win = d.w0;
@@ -441,50 +594,70 @@ __global__ void __launch_bounds__(kThreadsT, 1) taylor_kernel(const __grid_const
             for (int j = 0; j < d.m; ++j) {
                 const double coeff = d.coeff[j];
                 NormAcc nw, nf;
-                for (int r0 = rbeg; r0 < rend; r0 += R) {
-                    const int rows = min(R, rend - r0);
-                    double acc[CPT][CPLX ? 4 : 1];
-                    product_chunk<CPLX, S>(smem, d, win, ncols, r0, rows, acc);
-                    const int i = r0 + rr;
-                    const bool row_ok = rr < rows;
-                    double vw[CPT], vf[CPT];
+                for (int c0 = rbeg; c0 < rend; c0 += R) {
+                    const int rows = min(R, rend - c0);
+                    if (staging) {
+                        fence_async_global();
+                        bool ok = true;
+                        for (int t = 0; t < ktiles && ok; ++t) {
+                            if (t >= ahead) ok = st.put_a(c0, t * kt);
+                            if (ok) st.put_x(win, t * kt);
+                        }
+                        const int next = c0 + R < rend ? c0 + R : rbeg;
+                        for (int t = 0; t < ahead && ok; ++t) ok = st.put_a(next, t * kt);
+                    } else if (multiplying) {
+                        const int u = (rows + S::UNIT - 1) / S::UNIT, first = first_steps(u), second = threadIdx.x >> 7;
+                        multiply_dispatch<CPLX, S>(second ? u - first : first, smem, bars, ring, stages, stage_doubles,
+                                                   kt, units * S::UNIT, second ? first : 0, d.n, ncols, sY, L.err);
+                    }
+                    __syncthreads();
+#pragma unroll 2
+                    for (int b = 0; b < rows; b += RP) {
+                        const int r = b + rr, i = c0 + r;
+                        const bool row_ok = r < rows;
+                        double vw[CPT], vf[CPT];
 #pragma unroll
-                    for (int q = 0; q < CPT; ++q) {
-                        const int col = cs + q * S::SLOTS;
-                        vw[q] = 0.0;
-                        vf[q] = 0.0;
-                        if (row_ok && col < ncols) {
-                            const size_t pi = ((size_t)col * d.ldp + i) * es;
-                            if constexpr (CPLX) {
-                                // next = A work; work := Scale(next, coefficient) (ScaleInto, :441-452)
-                                const double yr = sub_rn(acc[q][0], acc[q][3]), yi = add_rn(acc[q][1], acc[q][2]);
-                                const double wr = mul_rn(yr, coeff), wi = mul_rn(yi, coeff);
-                                wout[pi] = wr;
-                                wout[pi + 1] = wi;
-                                // F += work (AddInto, :466-476)
-                                const double fr = add_rn(d.f[pi], wr), fi = add_rn(d.f[pi + 1], wi);
-                                d.f[pi] = fr;
-                                d.f[pi + 1] = fi;
-                                vw[q] = cabs_net(wr, wi);
-                                vf[q] = cabs_net(fr, fi);
-                            } else {
-                                const double w = mul_rn(acc[q][0], coeff);
-                                wout[pi] = w;
-                                const double fv = add_rn(d.f[pi], w);
-                                d.f[pi] = fv;
-                                vw[q] = fabs(w);
-                                vf[q] = fabs(fv);
+                        for (int q = 0; q < CPT; ++q) {
+                            const int col = cs + q * S::SLOTS;
+                            vw[q] = 0.0;
+                            vf[q] = 0.0;
+                            if (row_ok && col < ncols) {
+                                double* f = f_at(i, col);
+                                double* w = wout + ((size_t)i * S::COLS + col) * ES;
+                                const double* y = sY + (r * S::COLS + col) * ES;
+                                if constexpr (CPLX) {
+                                    // next = A work; work := Scale(next, coefficient) (ScaleInto, :441-452)
+                                    const double wr = mul_rn(y[0], coeff), wi = mul_rn(y[1], coeff);
+                                    *reinterpret_cast<double2*>(w) = make_double2(wr, wi);
+                                    // F += work (AddInto, :466-476)
+                                    const double fr = add_rn(f[0], wr), fi = add_rn(f[1], wi);
+                                    f[0] = fr;
+                                    f[1] = fi;
+                                    vw[q] = cabs_net(wr, wi);
+                                    vf[q] = cabs_net(fr, fi);
+                                } else {
+                                    const double wr = mul_rn(y[0], coeff);
+                                    w[0] = wr;
+                                    const double fv = add_rn(f[0], wr);
+                                    f[0] = fv;
+                                    vw[q] = fabs(wr);
+                                    vf[q] = fabs(fv);
+                                }
                             }
                         }
+                        const double sw = row_sum<S>(vw, ncols), sf = row_sum<S>(vf, ncols);
+                        if (row_ok) {
+                            nw.add(sw);
+                            nf.add(sf);
+                        }
                     }
-                    const double sw = row_sum<S>(vw, ncols), sf = row_sum<S>(vf, ncols);
-                    if (row_ok) {
-                        nw.add(sw);
-                        nf.add(sf);
-                    }
+                    if (c0 + R < rend) __syncthreads();  // the next chunk's products overwrite sY
                 }
-                if (!group_norms(d, rank, phase, L, nw, nf, s_red, s_nan, s_part, s_norm, &s_flag)) return;
-                const double c2 = s_norm[0], fnorm = s_norm[1];
+                if (!group_norms(d, rank, phase, L, nw, nf, sh, &bars.dead)) {
+                    if (staging) st.drain();
+                    return;
+                }
+                const double c2 = sh.norm[0], fnorm = sh.norm[1];
                 ++applications;
                 double* tmp = win;
                 win = wout;
@@ -498,7 +671,7 @@ __global__ void __launch_bounds__(kThreadsT, 1) taylor_kernel(const __grid_const
             }
             // F *= eta (ScaleInPlace, :455-464); work := F (CopyInto); c1 = ||work||_inf.
             NormAcc ne, unused;
-            for (int r0 = rbeg; r0 < rend; r0 += R) {
+            for (int r0 = rbeg; r0 < rend; r0 += RP) {
                 const int i = r0 + rr;
                 const bool row_ok = i < rend;
                 double v[CPT];
@@ -507,8 +680,8 @@ __global__ void __launch_bounds__(kThreadsT, 1) taylor_kernel(const __grid_const
                     const int col = cs + q * S::SLOTS;
                     v[q] = 0.0;
                     if (row_ok && col < ncols) {
-                        const size_t pi = ((size_t)col * d.ldp + i) * es;
-                        double re = d.f[pi], im = CPLX ? d.f[pi + 1] : 0.0;
+                        double* f = f_at(i, col);
+                        double re = f[0], im = CPLX ? f[1] : 0.0;
                         if (!d.eta_one) {
                             if constexpr (CPLX) {
                                 // Complex multiply (left = F, right = eta), .NET's order of terms.
@@ -519,24 +692,45 @@ __global__ void __launch_bounds__(kThreadsT, 1) taylor_kernel(const __grid_const
                             } else {
                                 re = mul_rn(re, d.eta_re);
                             }
-                            d.f[pi] = re;
-                            if (CPLX) d.f[pi + 1] = im;
+                            f[0] = re;
+                            if (CPLX) f[1] = im;
                         }
-                        win[pi] = re;
-                        if (CPLX) win[pi + 1] = im;
+                        double* w = win + ((size_t)i * S::COLS + col) * ES;
+                        w[0] = re;
+                        if (CPLX) w[1] = im;
                         v[q] = modulus<CPLX>(re, im);
                     }
                 }
                 const double rs = row_sum<S>(v, ncols);
                 if (row_ok) ne.add(rs);
             }
-            if (!group_norms(d, rank, phase, L, ne, unused, s_red, s_nan, s_part, s_norm, &s_flag)) return;
-            c1 = s_norm[0];
+            if (!group_norms(d, rank, phase, L, ne, unused, sh, &bars.dead)) {
+                if (staging) st.drain();
+                return;
+            }
+            c1 = sh.norm[0];
         }
         if (rank == 0 && threadIdx.x == 0) {
             d.out[0] = applications;
             d.out[1] = early;
         }
+        if (f_local)
+            for (int i = rbeg + rr; i < rend; i += RP)
+#pragma unroll
+                for (int q = 0; q < CPT; ++q) {
+                    const int col = cs + q * S::SLOTS;
+                    if (col < ncols)
+                        for (int z = 0; z < ES; ++z) d.f[((size_t)col * d.ldp + i) * ES + z] = f_at(i, col)[z];
+                }
+        // The tiles of A copied ahead for a product that never came.
+        if (staging) st.drain();
+        __syncthreads();
+        if (threadIdx.x == 0)
+            for (int i = 0; i < stages; ++i) {
+                mbar_inval(&bars.full[i]);
+                mbar_inval(&bars.empty[i]);
+            }
+        __syncthreads();
     }
 }
 
@@ -580,81 +774,99 @@ const int kEll = 2, kMaxPower = 8;
 
 template <bool CPLX, class S>
 void launch_taylor(Context& ctx, const TaylorLaunch& L, int grid) {
-    using T = Tiles<CPLX, S>;
-    TNS_CUDA(cudaFuncSetAttribute(taylor_kernel<CPLX, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::SMEM));
+    TNS_CUDA(cudaFuncSetAttribute(taylor_kernel<CPLX, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemT));
     void* args[] = {const_cast<TaylorLaunch*>(&L)};
     TNS_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(taylor_kernel<CPLX, S>), dim3(grid),
-                                         dim3(kThreadsT), args, T::SMEM, ctx.stream));
+                                         dim3(kThreadsT), args, kSmemT, ctx.stream));
     ctx.kernel_launches++;
 }
 
 template <bool CPLX, class S>
 int resident_ctas(Context& ctx) {
-    using T = Tiles<CPLX, S>;
-    TNS_CUDA(cudaFuncSetAttribute(taylor_kernel<CPLX, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::SMEM));
+    TNS_CUDA(cudaFuncSetAttribute(taylor_kernel<CPLX, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemT));
     int per_sm = 0;
-    TNS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, taylor_kernel<CPLX, S>, kThreadsT, T::SMEM));
+    TNS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, taylor_kernel<CPLX, S>, kThreadsT, kSmemT));
     if (per_sm < 1) fail(TNS_E_DEVICE, "the Taylor kernel cannot be resident on this device");
     return per_sm * ctx.num_sms;
 }
 
 // One kernel instance per (element type, layout, skip form); L null: only the
 // count of resident CTAs.
+// What the host needs of a launch's Shape.
+struct Layout {
+    int cols, unit, rows, lanes;  // panel pitch, rows per step, rows per box at most, resident CTAs
+};
+
+// One kernel instance per (element type, layout, skip form); L null: only its
+// Layout.
+template <bool CPLX, class S>
+Layout taylor_shape(Context& ctx, const TaylorLaunch* L, int grid) {
+    if (L) launch_taylor<CPLX, S>(ctx, *L, grid);
+    return Layout{S::COLS, S::UNIT, S::ROWS, L ? grid : resident_ctas<CPLX, S>(ctx)};
+}
+
+// Layouts by panel width: up to 4, 8, 16 and 32 columns.
 template <bool CPLX, bool SKIP>
-int taylor_dispatch(Context& ctx, int layout, const TaylorLaunch* L, int grid) {
-    using S8 = Shape<8, 1, SKIP>;
-    using S16 = Shape<16, 1, SKIP>;
-    using S16x2 = Shape<16, 2, SKIP>;
-    if (!L) return layout == 0 ? resident_ctas<CPLX, S8>(ctx) : layout == 1 ? resident_ctas<CPLX, S16>(ctx)
-                                                                              : resident_ctas<CPLX, S16x2>(ctx);
-    if (layout == 0) launch_taylor<CPLX, S8>(ctx, *L, grid);
-    else if (layout == 1) launch_taylor<CPLX, S16>(ctx, *L, grid);
-    else launch_taylor<CPLX, S16x2>(ctx, *L, grid);
-    return grid;
+Layout taylor_dispatch(Context& ctx, int ncols, const TaylorLaunch* L, int grid) {
+    if (ncols <= 4) return taylor_shape<CPLX, Shape<4, 1, 3, SKIP>>(ctx, L, grid);
+    if (ncols <= 8) return taylor_shape<CPLX, Shape<8, 1, 7, SKIP>>(ctx, L, grid);
+    if (ncols <= 16) return taylor_shape<CPLX, Shape<16, 1, 8, SKIP>>(ctx, L, grid);
+    return taylor_shape<CPLX, Shape<16, 2, 4, SKIP>>(ctx, L, grid);
 }
 
-int taylor(Context& ctx, bool cplx, bool skip, int layout, const TaylorLaunch* L, int grid) {
-    if (cplx) return skip ? taylor_dispatch<true, true>(ctx, layout, L, grid) : taylor_dispatch<true, false>(ctx, layout, L, grid);
-    return skip ? taylor_dispatch<false, true>(ctx, layout, L, grid) : taylor_dispatch<false, false>(ctx, layout, L, grid);
+Layout taylor(Context& ctx, bool cplx, bool skip, int ncols, const TaylorLaunch* L, int grid) {
+    if (cplx) return skip ? taylor_dispatch<true, true>(ctx, ncols, L, grid) : taylor_dispatch<true, false>(ctx, ncols, L, grid);
+    return skip ? taylor_dispatch<false, true>(ctx, ncols, L, grid) : taylor_dispatch<false, false>(ctx, ncols, L, grid);
 }
 
-// The list schedule: each matrix's width from its share of the work, then,
-// longest first, onto the lanes that free up earliest. Returns per-lane lists
-// of (matrix, rank) sorted by (start time, placement order).
+// The schedule: each matrix's width (CTAs) and rows per CTA, and the per-lane
+// lists of (matrix, rank) sorted by (start time, placement order).
 struct Sched {
     std::vector<int> width, rows_per;
     std::vector<int> offsets;
     std::vector<TaylorPlan> plan;
+    double makespan = 0.0;
 };
 
-Sched schedule(const std::vector<int>& n, const std::vector<double>& apps, int ncols, int lanes, int chunk_rows) {
-    const size_t cnt = n.size();
-    Sched sc;
-    sc.width.assign(cnt, 1);
-    sc.rows_per.assign(cnt, 8);
-    // Time model per application: n x (rows per CTA) x ncols element steps
-    // at `rate` per CTA, plus a barrier overhead for groups wider than one.
-    // (Measured on the sweep: widths in proportion to the work share beat
-    // rounding the rows per CTA up to whole chunks.)
-    const double rate = 1.0e10, bar_wide = 2.0e-6, bar_one = 0.5e-6;
-    (void)chunk_rows;
-    std::vector<double> work(cnt);
-    double total = 0.0;
-    for (size_t k = 0; k < cnt; ++k) {
-        work[k] = apps[k] * (double)n[k] * n[k] * ncols;
-        total += work[k];
+// A CTA's rows in the fewest chunks of up to `most` rows, evenly: a short
+// last chunk costs far more per row than a full one.
+int chunk_rows(int rows, int unit, int most) {
+    const int units = rows / unit, chunks = (rows + most - 1) / most;
+    return (units + chunks - 1) / chunks * unit;
+}
+
+// Seconds of one application on a CTA with `rows` rows: its FP64 instructions
+// (a product and a sum each, 2.2 cycles of a partition per warp), a floor of
+// one k's latency, and the norms and the barrier.
+double app_seconds(int n, int rows, bool cplx, int cpt, int unit, int most, bool wide) {
+    const int chunk = chunk_rows(rows, unit, most), chunks = (rows + chunk - 1) / chunk;
+    const double steps = (double)(chunk / unit) * cpt;
+    const double cycles = cplx ? std::max(42.0, 18.0 + 18.3 * steps) : std::max(42.0, 24.0 + 6.0 * steps);
+    return chunks * (n * cycles / 1.9e9 + 0.4e-6 * steps / cpt) + (wide ? 3.6e-6 : 1.2e-6);
+}
+
+// The widest row ranges with which every matrix ends within `limit` alone.
+void split_rows(const std::vector<int>& n, const std::vector<double>& apps, bool cplx, int cpt, int lanes, int unit,
+                int most, double limit, Sched& sc, std::vector<double>& dur) {
+    for (size_t k = 0; k < n.size(); ++k) {
+        const int units = (n[k] + unit - 1) / unit;
+        int lo = std::max(1, (units + lanes - 1) / lanes), hi = units;  // lo always taken, whatever its time
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) / 2;
+            if (apps[k] * app_seconds(n[k], mid * unit, cplx, cpt, unit, most, mid < units) <= limit) lo = mid;
+            else hi = mid - 1;
+        }
+        const int w = (units + lo - 1) / lo;
+        const int u = (units + w - 1) / w;  // the same width, evenly
+        sc.rows_per[k] = u * unit;
+        sc.width[k] = (units + u - 1) / u;
+        dur[k] = apps[k] * app_seconds(n[k], u * unit, cplx, cpt, unit, most, sc.width[k] > 1);
     }
-    std::vector<double> dur(cnt);
-    for (size_t k = 0; k < cnt; ++k) {
-        const int max_w = std::max(1, std::min(lanes, (n[k] + 7) / 8));
-        int w = total > 0.0 ? (int)std::lround(lanes * work[k] / total) : 1;
-        w = std::clamp(w, 1, max_w);
-        int rp = round_up((n[k] + w - 1) / w, 8);
-        w = (n[k] + rp - 1) / rp;  // no rank without rows
-        sc.width[k] = w;
-        sc.rows_per[k] = rp;
-        dur[k] = apps[k] * ((double)n[k] * rp * ncols / rate + (w > 1 ? bar_wide : bar_one));
-    }
+}
+
+// Longest first, onto the lanes that free up earliest.
+void place(Sched& sc, const std::vector<double>& dur, int lanes) {
+    const size_t cnt = dur.size();
     std::vector<int> order(cnt);
     std::iota(order.begin(), order.end(), 0);
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return dur[x] > dur[y]; });
@@ -666,6 +878,7 @@ Sched schedule(const std::vector<int>& n, const std::vector<double>& apps, int n
     std::vector<std::vector<Entry>> per_lane(lanes);
     std::vector<int> idx(lanes);
     int seq = 0;
+    sc.makespan = 0.0;
     for (int k : order) {
         const int w = sc.width[k];
         std::iota(idx.begin(), idx.end(), 0);
@@ -677,16 +890,46 @@ Sched schedule(const std::vector<int>& n, const std::vector<double>& apps, int n
             per_lane[idx[r]].push_back(Entry{start, seq, k, r});
             free_at[idx[r]] = start + dur[k];
         }
+        sc.makespan = std::max(sc.makespan, start + dur[k]);
         ++seq;
     }
     sc.offsets.assign(lanes + 1, 0);
+    sc.plan.clear();
     for (int l = 0; l < lanes; ++l) {
         auto& v = per_lane[l];
         std::sort(v.begin(), v.end(), [](const Entry& x, const Entry& y) { return x.start < y.start || (x.start == y.start && x.seq < y.seq); });
         sc.offsets[l + 1] = sc.offsets[l] + (int)v.size();
         for (auto& e : v) sc.plan.push_back(TaylorPlan{e.matrix, e.rank});
     }
-    return sc;
+}
+
+// Widths from a limit on each matrix's own time: the smallest limit with
+// which all of them run side by side, found by bisection, and shorter ones,
+// with which the later matrices follow on lanes that earlier ones left; the
+// limit whose list schedule ends first is taken.
+Sched schedule(const std::vector<int>& n, const std::vector<double>& apps, bool cplx, int cpt, int lanes, int unit, int most) {
+    const size_t cnt = n.size();
+    Sched sc, best;
+    sc.width.assign(cnt, 1);
+    sc.rows_per.assign(cnt, unit);
+    std::vector<double> dur(cnt);
+    double longest = 0.0;  // with one CTA each
+    for (size_t k = 0; k < cnt; ++k)
+        longest = std::max(longest, apps[k] * app_seconds(n[k], (n[k] + unit - 1) / unit * unit, cplx, cpt, unit, most, false));
+    double lo = 0.0, hi = longest;
+    for (int it = 0; it < 24; ++it) {
+        const double mid = 0.5 * (lo + hi);
+        split_rows(n, apps, cplx, cpt, lanes, unit, most, mid, sc, dur);
+        if (std::accumulate(sc.width.begin(), sc.width.end(), 0) <= lanes) hi = mid;
+        else lo = mid;
+    }
+    for (double f : {1.0, 0.8, 0.6, 0.4, 0.2}) {
+        split_rows(n, apps, cplx, cpt, lanes, unit, most, hi * f, sc, dur);
+        place(sc, dur, lanes);
+        if (f == 1.0 || sc.makespan < best.makespan) best = sc;
+        if (cnt == 1) break;
+    }
+    return best;
 }
 
 }  // namespace
@@ -787,16 +1030,13 @@ void expmv_batch(Context& ctx, const std::vector<const DMat*>& as, const std::ve
             expmv_taylor_host(ctx, sh[k], *bs[k], t, ms[k], ss[k], eta_re[k], eta_im[k], results[k], &infos[k]);
         return;
     }
-    // Layout: 8 slots x 64 rows for up to 8 columns, 16 x 32 for up to 16,
-    // 16 x 32 with two columns per slot for up to 32.
-    const int layout = ncols <= 8 ? 0 : ncols <= 16 ? 1 : 2;
     // The explicit zero skip only when some operator has a non-finite entry
     // (its parameters can still be finite: a nilpotent shifted operator has
     // d(p) = 0 for p >= 2).
     bool skip = false;
     for (size_t k = 0; k < cnt; ++k)
         if (!std::isfinite(one_norm[k])) skip = true;
-    const int lanes = taylor(ctx, cplx, skip, layout, nullptr, 0);
+    const Layout lay = taylor(ctx, cplx, skip, ncols, nullptr, 0);
 
     std::vector<int> orders(cnt);
     std::vector<double> apps(cnt);
@@ -804,41 +1044,44 @@ void expmv_batch(Context& ctx, const std::vector<const DMat*>& as, const std::ve
         orders[k] = as[k]->rows;
         apps[k] = std::max(1.0, (double)ms[k] * ss[k]);
     }
-    Sched sc = schedule(orders, apps, ncols, lanes, layout == 0 ? 64 : 32);
+    Sched sc = schedule(orders, apps, cplx, ncols > 16 ? 2 : 1, lay.lanes, lay.unit, lay.rows);
 
-    std::vector<DMat> w0(cnt), w1(cnt);
-    size_t partial_doubles = 0;
+    size_t panel_bytes = 0, slot_words = 0;
     for (size_t k = 0; k < cnt; ++k) {
         results[k] = DMat(ctx, orders[k], ncols, cplx, "the exponential action");
-        w0[k] = DMat(ctx, orders[k], ncols, cplx, "a Taylor work panel");
-        w1[k] = DMat(ctx, orders[k], ncols, cplx, "a Taylor work panel");
-        partial_doubles += 4 * (size_t)sc.width[k];
+        panel_bytes += 2 * (size_t)orders[k] * lay.cols * as[k]->esz();
+        slot_words += 6 * (size_t)sc.width[k];
     }
-    const size_t state_bytes = sizeof(unsigned long long) * (cnt + 1) + sizeof(int) * 2 * cnt;
+    DBuf panels(ctx, panel_bytes);
+    const size_t state_bytes = sizeof(unsigned long long) + sizeof(int) * 2 * cnt;
     DBuf state(ctx, state_bytes);
     TNS_CUDA(cudaMemsetAsync(state.p, 0, state_bytes, ctx.stream));
-    unsigned long long* bars = state.as<unsigned long long>();
-    int* outs = reinterpret_cast<int*>(bars + cnt + 1);
-    DBuf partials(ctx, sizeof(double) * std::max<size_t>(partial_doubles, 1));
+    int* outs = reinterpret_cast<int*>(state.as<unsigned long long>() + 1);
+    DBuf slots(ctx, sizeof(unsigned long long) * slot_words);
+    TNS_CUDA(cudaMemsetAsync(slots.p, 0xff, sizeof(unsigned long long) * slot_words, ctx.stream));
     DBuf dcoeff(ctx, sizeof(double) * std::max<size_t>(coeffs.size(), 1));
     if (!coeffs.empty())
         TNS_CUDA(cudaMemcpyAsync(dcoeff.p, coeffs.data(), sizeof(double) * coeffs.size(), cudaMemcpyHostToDevice, ctx.stream));
     std::vector<TaylorDesc> descs(cnt);
-    size_t poff = 0;
+    std::vector<CUtensorMap> maps(cnt);
+    double* panel = panels.as<double>();
+    unsigned long long* slot = slots.as<unsigned long long>();
     for (size_t k = 0; k < cnt; ++k) {
         TaylorDesc& d = descs[k];
-        d.a = sh[k].p;
-        d.lda = sh[k].ld();
         d.b = bs[k]->p;
         d.ldb = bs[k]->ld();
         d.f = results[k].p;
-        d.w0 = w0[k].p;
-        d.w1 = w1[k].p;
+        const size_t es = cplx ? 2 : 1, panel_doubles = (size_t)orders[k] * lay.cols * es;
+        d.w0 = panel;
+        d.w1 = panel + panel_doubles;
+        panel += 2 * panel_doubles;
         d.ldp = results[k].ld();
         d.coeff = dcoeff.as<double>() + coeff_off[k];
-        d.partials = partials.as<double>() + poff;
-        poff += 4 * (size_t)sc.width[k];
-        d.bar = bars + k;
+        d.slots = slot;
+        slot += 6 * (size_t)sc.width[k];
+        d.chunk = chunk_rows(sc.rows_per[k], lay.unit, lay.rows);
+        encode_map_2d(&maps[k], sh[k].p, es * orders[k], orders[k], (uint64_t)sh[k].ld() * sh[k].esz(),
+                      (uint32_t)(es * d.chunk), tile_k(d.chunk, lay.cols));
         d.out = outs + 2 * k;
         d.n = orders[k];
         d.m = ms[k];
@@ -855,8 +1098,9 @@ void expmv_batch(Context& ctx, const std::vector<const DMat*>& as, const std::ve
     L.plan_off = static_cast<const int*>(ctx.upload(sc.offsets.data(), sizeof(int) * sc.offsets.size()));
     L.ncols = ncols;
     L.err = ctx.d_err;
-    L.progress = bars + cnt;
-    taylor(ctx, cplx, skip, layout, &L, lanes);
+    L.progress = state.as<unsigned long long>();
+    L.maps = static_cast<const CUtensorMap*>(ctx.upload(maps.data(), sizeof(CUtensorMap) * cnt));
+    taylor(ctx, cplx, skip, ncols, &L, lay.lanes);
     std::vector<int> h(2 * cnt);
     TNS_CUDA(cudaMemcpyAsync(h.data(), outs, sizeof(int) * 2 * cnt, cudaMemcpyDeviceToHost, ctx.stream));
     ctx.sync();

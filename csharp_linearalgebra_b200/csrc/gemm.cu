@@ -581,6 +581,31 @@ __global__ void __launch_bounds__(256) slab_fold_kernel(const __grid_constant__ 
 // Host side
 // ---------------------------------------------------------------------------
 
+// A 2-D double-precision TMA descriptor: `rows` x `cols` doubles, column
+// stride `ld_bytes`, boxes of box_rows x box_cols, zero fill outside.
+void encode_map_2d(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint64_t ld_bytes,
+                uint32_t box_rows, uint32_t box_cols) {
+    cuuint64_t dims[2] = {rows, cols};
+    cuuint64_t strides[1] = {ld_bytes};
+    cuuint32_t box[2] = {box_rows, box_cols};
+    cuuint32_t elem[2] = {1, 1};
+    // The driver's encoder, looked up through the runtime so that the library
+    // loads (and its host-only entry points work) where no driver is present.
+    static PFN_cuTensorMapEncodeTiled_v12000 encode = [] {
+        void* fn = nullptr;
+        cudaDriverEntryPointQueryResult q{};
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess)
+            fn = nullptr;
+        return reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
+    }();
+    if (!encode) fail(TNS_E_DEVICE, "the CUDA driver does not provide cuTensorMapEncodeTiled");
+    CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, const_cast<void*>(base), dims, strides, box, elem,
+                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                        CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) fail(TNS_E_DEVICE, "TMA descriptor encoding failed (CUresult " + std::to_string((int)r) + ")");
+}
+
 namespace {
 
 using RealBig = GemmCfg<false, 4, 2, 4>;    // 128 x 128 tiles, 8 math warps
@@ -606,38 +631,13 @@ void check_register_split() {
     }
 }
 
-// A 2-D double-precision TMA descriptor: `rows` x `cols` doubles, column
-// stride `ld_bytes`, boxes of box_rows x box_cols, zero fill outside.
-void encode_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint64_t ld_bytes,
-                uint32_t box_rows, uint32_t box_cols) {
-    cuuint64_t dims[2] = {rows, cols};
-    cuuint64_t strides[1] = {ld_bytes};
-    cuuint32_t box[2] = {box_rows, box_cols};
-    cuuint32_t elem[2] = {1, 1};
-    // The driver's encoder, looked up through the runtime so that the library
-    // loads (and its host-only entry points work) where no driver is present.
-    static PFN_cuTensorMapEncodeTiled_v12000 encode = [] {
-        void* fn = nullptr;
-        cudaDriverEntryPointQueryResult q{};
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q) != cudaSuccess ||
-            q != cudaDriverEntryPointSuccess)
-            fn = nullptr;
-        return reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
-    }();
-    if (!encode) fail(TNS_E_DEVICE, "the CUDA driver does not provide cuTensorMapEncodeTiled");
-    CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, const_cast<void*>(base), dims, strides, box, elem,
-                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                        CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) fail(TNS_E_DEVICE, "TMA descriptor encoding failed (CUresult " + std::to_string((int)r) + ")");
-}
-
 // Descriptors of one problem's operands for configuration Cfg.
 template <class Cfg>
 GemmMaps encode_maps(const GemmProblem& p) {
     GemmMaps m;
-    encode_map(&m.a, p.A, (uint64_t)Cfg::DPE * p.M, (uint64_t)p.K, (uint64_t)p.lda * Cfg::ESZ,
+    encode_map_2d(&m.a, p.A, (uint64_t)Cfg::DPE * p.M, (uint64_t)p.K, (uint64_t)p.lda * Cfg::ESZ,
                Cfg::DPE * Cfg::LDA_S, Cfg::BK);
-    encode_map(&m.b, p.B, (uint64_t)Cfg::DPE * p.K, (uint64_t)p.N, (uint64_t)p.ldb * Cfg::ESZ,
+    encode_map_2d(&m.b, p.B, (uint64_t)Cfg::DPE * p.K, (uint64_t)p.N, (uint64_t)p.ldb * Cfg::ESZ,
                Cfg::DPE * Cfg::LDB_S, Cfg::BN);
     return m;
 }

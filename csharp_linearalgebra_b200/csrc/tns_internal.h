@@ -14,6 +14,8 @@
 
 #include "../../include/tensile_b200.h"
 
+struct CUtensorMap_st;
+
 namespace tns {
 
 // Thrown inside the library, caught at the C ABI and mapped to a status code.
@@ -208,6 +210,10 @@ void copy_out(Context& ctx, const DMat& src, double* dst, int ld, bool dst_on_de
 // The same on another stream (the caller orders it after the producer).
 void copy_out_on(cudaStream_t stream, const DMat& src, double* dst, int ld, bool dst_on_device);
 void copy_dmat(Context& ctx, DMat& dst, const DMat& src);
+// A 2-D double-precision TMA descriptor (gemm.cu): `rows` x `cols` doubles,
+// column stride `ld_bytes`, boxes of box_rows x box_cols, zero fill outside.
+void encode_map_2d(CUtensorMap_st* map, const void* base, uint64_t rows, uint64_t cols, uint64_t ld_bytes,
+                   uint32_t box_rows, uint32_t box_cols);
 
 // ---- GEMM (gemm.cu) --------------------------------------------------------
 void gemm_grouped(Context& ctx, std::vector<GemmProblem>& probs, bool cplx);
