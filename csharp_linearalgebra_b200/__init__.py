@@ -324,14 +324,15 @@ class Workspace:
     def factor_lu(self, a, block_size: int = 0) -> "LuDecomposition":
         """P*A = L*U with partial pivoting (Workspace.FactorLu)."""
         cplx = np.iscomplexobj(a)
-        f = _fortran(a, cplx).copy(order="F")
-        if f.ndim != 2:
+        a = _fortran(a, cplx)
+        if a.ndim != 2:
             raise ValueError("a matrix is required")
-        m, n = f.shape
+        m, n = a.shape
+        f = np.empty((m, n), dtype=a.dtype, order="F")
         piv = np.zeros(min(m, n), dtype=np.int32)
         info = N.LuInfo()
-        self._call("tns_zgetrf" if cplx else "tns_dgetrf", m, n, _p(f), _ld(f), int(block_size), _p(piv),
-                   C.byref(info))
+        self._call("tns_zgetrf_to" if cplx else "tns_dgetrf_to", m, n, _p(a), _ld(a), _p(f), _ld(f), int(block_size),
+                   _p(piv), C.byref(info))
         return LuDecomposition(self, f, piv, info)
 
     # -- estimation ---------------------------------------------------------

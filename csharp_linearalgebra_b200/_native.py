@@ -84,6 +84,8 @@ SIGNATURES = {
     "tns_znorm": (_I, [_P, _CH, _I, _I, _P, _I, C.POINTER(_D)]),
     "tns_dgetrf": (_I, [_P, _I, _I, _P, _I, _I, _P, C.POINTER(LuInfo)]),
     "tns_zgetrf": (_I, [_P, _I, _I, _P, _I, _I, _P, C.POINTER(LuInfo)]),
+    "tns_dgetrf_to": (_I, [_P, _I, _I, _P, _I, _P, _I, _I, _P, C.POINTER(LuInfo)]),
+    "tns_zgetrf_to": (_I, [_P, _I, _I, _P, _I, _P, _I, _I, _P, C.POINTER(LuInfo)]),
     "tns_dgetrs": (_I, [_P, _I, _I, _P, _I, _P, _I, _P, _I, _I]),
     "tns_zgetrs": (_I, [_P, _I, _I, _P, _I, _P, _I, _P, _I, _I]),
     **{name: (_I, [_P, _I, _I, _P, _I, _P, _I]) for name in (

@@ -17,7 +17,7 @@ LIB = os.path.join(HERE, "libtensile_b200.so")
 OBJ = os.path.join(HERE, "_build")
 
 SOURCES = ["context.cu", "gemm.cu", "blas1.cu", "lu.cu", "lu_panel.cu", "subst_cols.cu", "subst_left.cu", "estimate.cu", "algos.cu", "expm_batched.cu", "expmv_batched.cu", "capi.cu",
-           "noalloc.cu",
+           "noalloc.cu", "host_copy.cu",
            "ozaki.cu", "frechet.cu"]
 
 NVCC_FLAGS = [

@@ -145,9 +145,12 @@ int norm_entry(tns_context* c, bool cplx, char kind, int m, int n, const double*
     });
 }
 
-int getrf_entry(tns_context* c, bool cplx, int m, int n, double* a, int lda, int nb, int* pivots, tns_lu_info* info) {
+// The factors go to f (which may be a).
+int getrf_entry(tns_context* c, bool cplx, int m, int n, const double* a, int lda, double* f, int ldf, int nb, int* pivots,
+                tns_lu_info* info) {
     return guarded(c, [&](Context& ctx) {
         check_operand(a, m, n, lda, "A");
+        check_operand(f, m, n, ldf, "the factors");
         int limit = std::min(m, n);
         require(pivots != nullptr || limit == 0, TNS_E_NULL, "pivots is null");
         tns_lu_info local{};
@@ -161,7 +164,7 @@ int getrf_entry(tns_context* c, bool cplx, int m, int n, double* a, int lda, int
         tns::LuResult r = tns::getrf(ctx, A, m, n, nb, piv.as<int>());
         std::vector<int> hp(limit);
         TNS_CUDA(cudaMemcpyAsync(hp.data(), piv.p, sizeof(int) * limit, cudaMemcpyDeviceToHost, ctx.stream));
-        tns::copy_out(ctx, A, a, lda, false);
+        tns::copy_out(ctx, A, f, ldf, false);
         ctx.sync();
         std::memcpy(pivots, hp.data(), sizeof(int) * limit);
         out->singular_column = r.singular_column;
@@ -850,10 +853,18 @@ int tns_znorm(tns_context* c, char kind, int m, int n, const double* a, int lda,
 }
 
 int tns_dgetrf(tns_context* c, int m, int n, double* a, int lda, int nb, int* pivots, tns_lu_info* info) {
-    return getrf_entry(c, false, m, n, a, lda, nb, pivots, info);
+    return getrf_entry(c, false, m, n, a, lda, a, lda, nb, pivots, info);
 }
 int tns_zgetrf(tns_context* c, int m, int n, double* a, int lda, int nb, int* pivots, tns_lu_info* info) {
-    return getrf_entry(c, true, m, n, a, lda, nb, pivots, info);
+    return getrf_entry(c, true, m, n, a, lda, a, lda, nb, pivots, info);
+}
+int tns_dgetrf_to(tns_context* c, int m, int n, const double* a, int lda, double* f, int ldf, int nb, int* pivots,
+                  tns_lu_info* info) {
+    return getrf_entry(c, false, m, n, a, lda, f, ldf, nb, pivots, info);
+}
+int tns_zgetrf_to(tns_context* c, int m, int n, const double* a, int lda, double* f, int ldf, int nb, int* pivots,
+                  tns_lu_info* info) {
+    return getrf_entry(c, true, m, n, a, lda, f, ldf, nb, pivots, info);
 }
 int tns_dgetrs(tns_context* c, int n, int nrhs, const double* lu, int lda, const int* pivots, int singular_column,
                double* b, int ldb, int adjoint) {

@@ -76,6 +76,7 @@ Context::~Context() {
             cudaEventDestroy(pr.second);
         }
     for (auto e : event_pool) cudaEventDestroy(e);
+    copier.reset();
     if (split_scratch) cudaFree(split_scratch);
     if (h_ring) cudaFreeHost(h_ring);
     if (d_ring) cudaFree(d_ring);
@@ -223,9 +224,28 @@ DBuf::~DBuf() {
     if (p && ctx) cudaFreeAsync(p, ctx->stream);
 }
 
+HostCopier* Context::host_copier(const void* host, size_t bytes) {
+    if (bytes < HostCopier::kLeast || concurrent) return nullptr;
+    // Pinned, managed and device memory passed as a host operand go as they are.
+    cudaPointerAttributes at{};
+    if (cudaPointerGetAttributes(&at, host) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    if (at.type != cudaMemoryTypeUnregistered) return nullptr;
+    if (!copier) copier = std::make_unique<HostCopier>(device);
+    return copier->usable() ? copier.get() : nullptr;
+}
+
 void copy_in(Context& ctx, DMat& dst, const double* src, int ld, bool src_on_device) {
     if (dst.rows == 0 || dst.cols == 0) return;
     size_t esz = dst.esz();
+    if (!src_on_device)
+        if (HostCopier* h = ctx.host_copier(src, (size_t)dst.rows * dst.cols * esz)) {
+            TNS_CUDA(h->to_device(ctx.stream, reinterpret_cast<char*>(dst.p), dst.ld(), reinterpret_cast<const char*>(src),
+                                  ld, dst.rows, dst.cols, esz));
+            return;
+        }
     TNS_CUDA(cudaMemcpy2DAsync(dst.p, (size_t)dst.ld() * esz, src, (size_t)ld * esz, (size_t)dst.rows * esz, dst.cols,
                                src_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, ctx.stream));
 }
@@ -238,6 +258,12 @@ void copy_out_on(cudaStream_t stream, const DMat& src, double* dst, int ld, bool
 }
 
 void copy_out(Context& ctx, const DMat& src, double* dst, int ld, bool dst_on_device) {
+    if (!dst_on_device && src.rows && src.cols)
+        if (HostCopier* h = ctx.host_copier(dst, (size_t)src.rows * src.cols * src.esz())) {
+            TNS_CUDA(h->to_host(ctx.stream, reinterpret_cast<char*>(dst), ld, reinterpret_cast<const char*>(src.p),
+                                src.ld(), src.rows, src.cols, src.esz()));
+            return;
+        }
     copy_out_on(ctx.stream, src, dst, ld, dst_on_device);
 }
 

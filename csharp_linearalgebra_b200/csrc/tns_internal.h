@@ -3,6 +3,8 @@
 // the launchers of the sm_100a kernels.
 #pragma once
 
+#include "host_copy.h"
+
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -139,6 +141,11 @@ struct Context {
     // still running on `stream` (created on first use).
     cudaStream_t copy_stream = nullptr;
     cudaStream_t copies();
+
+    // Large copies of pageable host memory (made at the first of them). Null
+    // for batch workers, whose copies overlap one another already.
+    std::unique_ptr<HostCopier> copier;
+    HostCopier* host_copier(const void* host, size_t bytes);
 
     // Batched work runs on worker contexts (one host thread and one stream
     // each), created on first use, so that independent matrices overlap on

@@ -143,6 +143,11 @@ int tns_dgetrf(tns_context* ctx, int m, int n, double* a, int lda, int nb, int* 
                tns_lu_info* info);
 int tns_zgetrf(tns_context* ctx, int m, int n, double* a, int lda, int nb, int* pivots,
                tns_lu_info* info);
+/* The same with the factors written to f and a left as it is. */
+int tns_dgetrf_to(tns_context* ctx, int m, int n, const double* a, int lda, double* f, int ldf,
+                  int nb, int* pivots, tns_lu_info* info);
+int tns_zgetrf_to(tns_context* ctx, int m, int n, const double* a, int lda, double* f, int ldf,
+                  int nb, int* pivots, tns_lu_info* info);
 
 /* Solve A X = B (adjoint = 0) or A^H X = B (adjoint = 1) in place from a
  * factorization; TNS_E_SINGULAR when singular_column >= 0.
