@@ -163,14 +163,24 @@ __global__ void col_abs_sums_kernel(const __grid_constant__ Batch<SumDesc> b) {
     if (lane == 0) d.out[j] = sum;
 }
 
-// One thread per row: sequential sum over columns in column order.
+// One thread per row: sequential sum over columns in column order, sixteen
+// loads ahead of their additions (one load at a time, each addition waited for
+// memory: 948 us for 4096 x 4096).
 template <bool CPLX>
 __global__ void row_abs_sums_kernel(const __grid_constant__ Batch<SumDesc> b) {
     const SumDesc& d = batch_item(b, blockIdx.y);
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= d.m) return;
     double sum = 0.0;
-    for (int j = 0; j < d.n; ++j) sum = add_rn(sum, mag(d.a, (size_t)j * d.ld + i, CPLX));
+    int j = 0;
+    for (; j + 16 <= d.n; j += 16) {
+        double v[16];
+#pragma unroll
+        for (int u = 0; u < 16; ++u) v[u] = mag(d.a, (size_t)(j + u) * d.ld + i, CPLX);
+#pragma unroll
+        for (int u = 0; u < 16; ++u) sum = add_rn(sum, v[u]);
+    }
+    for (; j < d.n; ++j) sum = add_rn(sum, mag(d.a, (size_t)j * d.ld + i, CPLX));
     d.out[i] = sum;
 }
 

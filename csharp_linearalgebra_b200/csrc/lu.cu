@@ -27,6 +27,7 @@
 
 #include "batch.cuh"
 #include "device_util.cuh"
+#include "divide.cuh"
 #include "lu_panel.h"
 #include "subst_cols.h"
 #include "subst_left.h"
@@ -1716,6 +1717,12 @@ void getrs(Context& ctx, const DMat& lu, const int* d_piv, DMat& b, int nrhs, bo
     getrs_batch(ctx, items, adjoint);
 }
 
+// The precision form's solves of up to this many columns take the one-launch
+// solve (2.1 ms for 64 columns of 4096 rows, 4.2 by blocks and updates). A
+// whole solve, n = 4096: 53.97 ms by blocks and 43.93 in one launch with 64
+// columns, 61.8 and 57.5 with 512, 72.3 and 79.1 with 1024.
+constexpr int kOneLaunchCols = 512;
+
 void getrs_free_order(Context& ctx, const DMat& lu, const int* d_piv, DMat& b, int nrhs, bool adjoint) {
     const int n = lu.rows;
     if (n == 0 || nrhs == 0) return;
@@ -1903,8 +1910,8 @@ void mixed_trailing(Context& ctx, DMat& a, int j, int w, int moduli) {
     // U12 := L11^-1 A12: 64-row unit-lower blocks, DMMA updates below each.
     for (int b0 = 0; b0 < w; b0 += 64) {
         const int bw = std::min(64, w - b0);
-        std::vector<TrsmDesc> t{TrsmDesc{a.at(j + b0, j + b0), ld, a.at(j + b0, j + w), ld, bw, rest, 1, 1, 0}};
-        launch_trsm(ctx, cplx, t);
+        std::vector<PanelRowsDesc> u{PanelRowsDesc{a.p, ld, j + w, j + w + rest, nullptr, j + b0, bw, 0, 1, 0}};
+        launch_panel_rows(ctx, cplx, u);
         if (b0 + bw < w) {
             GemmProblem p{};
             p.A = a.at(j + b0 + bw, j + b0);
@@ -2010,7 +2017,11 @@ void gesv_mixed_pivoted(Context& ctx, const DMat& a, const DMat& b, DMat& x, int
     copy_dmat(ctx, x, b);
     // The precision form's solves have no reference order to keep: blocked
     // triangular solves with DMMA updates.
-    getrs_free_order(ctx, f, piv.as<int>(), x, nrhs, false);
+    auto lu_solve = [&](DMat& m) {
+        if (nrhs <= kOneLaunchCols) getrs(ctx, f, piv.as<int>(), m, nrhs, false);
+        else getrs_free_order(ctx, f, piv.as<int>(), m, nrhs, false);
+    };
+    lu_solve(x);
     const double ainf = norminf(ctx, a);
     const std::vector<double> bmax = col_absmax(ctx, b);
     DMat r(ctx, n, nrhs, cplx, "the refinement residual");
@@ -2028,7 +2039,7 @@ void gesv_mixed_pivoted(Context& ctx, const DMat& a, const DMat& b, DMat& x, int
         info.backward_error = berr;
         if (berr <= 4.0 * 1.1102230246251565e-16 || it >= max_iter || !(berr < 0.5 * prev)) break;
         prev = berr;
-        getrs_free_order(ctx, f, piv.as<int>(), r, nrhs, false);
+        lu_solve(r);
         std::vector<EwDesc> add{ew_add_scaled(x, r, 1.0)};
         ew_batch(ctx, add);
         info.iterations++;
@@ -2166,71 +2177,161 @@ __device__ __forceinline__ void stage_block(Z* s, const double* src, int ld, int
 // The w x w diagonal block (w <= 64) factored in place without pivoting,
 // L unit lower and U upper; an exactly zero pivot records its column (atomic
 // minimum into flag) and the factorization goes on in inf/NaN.
+//
+// One CTA, 64 dependent steps: their latency is all there is to it. Thread
+// (r, g) holds row r's columns g, g + 4, ...; a step reads the published
+// column k and row k, divides in every thread, updates and publishes column
+// and row k + 1: one barrier, one division, selects instead of branches. Four
+// steps on, the first register holds a finished column: it is stored and the
+// others move up, so that no register is indexed by k. 24 us for 64 x 64 (the
+// block in shared memory, two barriers a step and every element located by a
+// division: 56; branches in place of the selects: 40).
+template <bool CPLX, int NQ>
+__device__ __forceinline__ void nopiv_diag_steps(Z (&v)[kNopivBlock / 4], Z (&scol)[2][kNopivBlock],
+                                                 Z (&srow)[2][kNopivBlock], double* a, int ld, int w, int col0,
+                                                 int* flag) {
+    constexpr int ES = CPLX ? 2 : 1, Q = kNopivBlock / 4;
+    const int r = threadIdx.x & 63, g = threadIdx.x >> 6;
+    // NQ registers, then NQ - 1, ... are live; four at a time share code.
+    for (int q0 = Q - NQ; q0 < Q - NQ + 4 && 4 * q0 < w; ++q0) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int k = 4 * q0 + i;
+            const Z* row = srow[i & 1] + 4 * q0 + g;
+            const Z piv = srow[i & 1][k];
+            Z u[NQ];
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) u[q] = row[4 * (q0 + q < Q ? q : 0)];
+            const Z l = div_el<CPLX>(scol[i & 1][r], piv);
+            const bool below = r > k;
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) {
+                const Z t = sub_prod<CPLX>(v[q], l, u[q]);
+                const bool take = below && (q > 0 || g > i);
+                v[q].re = take ? t.re : v[q].re;
+                if (CPLX) v[q].im = take ? t.im : v[q].im;
+            }
+            const bool own = below && g == i;
+            v[0].re = own ? l.re : v[0].re;
+            if (CPLX) v[0].im = own ? l.im : v[0].im;
+            if (k + 1 < kNopivBlock) {
+                if (g == (i + 1) % 4) scol[(i + 1) & 1][r] = i < 3 ? v[0] : v[1];
+                if (r == k + 1)
+#pragma unroll
+                    for (int q = 0; q < NQ; ++q)
+                        if (q0 + q < Q) srow[(i + 1) & 1][4 * (q0 + q) + g] = v[q];
+            }
+            if (threadIdx.x == 0 && k < w && piv.re == 0.0 && piv.im == 0.0) atomicMin(flag, col0 + k);
+            __syncthreads();
+        }
+        const int c = 4 * q0 + g;
+        if (r < w && c < w) store_el<CPLX>(a + ((size_t)c * ld + r) * ES, v[0]);
+#pragma unroll
+        for (int q = 0; q + 1 < NQ; ++q) v[q] = v[q + 1];
+    }
+}
+
 template <bool CPLX>
 __global__ void __launch_bounds__(256) lu_nopiv_diag_kernel(double* a, int ld, int w, int col0, int* flag) {
-    constexpr int ES = CPLX ? 2 : 1;
-    extern __shared__ __align__(16) unsigned char nopiv_smem[];
-    Z* s = reinterpret_cast<Z*>(nopiv_smem);  // s[c * kNopivLd + r]
-    stage_block<CPLX>(s, a, ld, w, w, false);
+    constexpr int ES = CPLX ? 2 : 1, Q = kNopivBlock / 4;
+    __shared__ Z scol[2][kNopivBlock], srow[2][kNopivBlock];
+    const int r = threadIdx.x & 63, g = threadIdx.x >> 6;
+    Z v[Q];
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+        // Past w the identity, whose steps change nothing.
+        const int c = 4 * q + g;
+        v[q] = r < w && c < w ? load_el<CPLX>(a + ((size_t)c * ld + r) * ES) : Z{r == c ? 1.0 : 0.0, 0.0};
+    }
+    if (g == 0) scol[0][r] = v[0];
+    if (r == 0)
+#pragma unroll
+        for (int q = 0; q < Q; ++q) srow[0][4 * q + g] = v[q];
     __syncthreads();
-    for (int k = 0; k < w; ++k) {
-        const Z piv = s[k * kNopivLd + k];
-        if (threadIdx.x == 0 && piv.re == 0.0 && piv.im == 0.0) atomicMin(flag, col0 + k);
-        for (int r = k + 1 + threadIdx.x; r < w; r += blockDim.x)
-            s[k * kNopivLd + r] = div_el<CPLX>(s[k * kNopivLd + r], piv);
-        __syncthreads();
-        const int m = w - k - 1;
-        for (int e = threadIdx.x; e < m * m; e += blockDim.x) {
-            const int r = k + 1 + e % m, c = k + 1 + e / m;
-            s[c * kNopivLd + r] = sub_prod<CPLX>(s[c * kNopivLd + r], s[k * kNopivLd + r], s[c * kNopivLd + k]);
-        }
-        __syncthreads();
-    }
-    for (int e = threadIdx.x; e < w * w; e += blockDim.x) {
-        const int r = e % w, c = e / w;
-        store_el<CPLX>(a + ((size_t)c * ld + r) * ES, s[c * kNopivLd + r]);
-    }
+    nopiv_diag_steps<CPLX, 16>(v, scol, srow, a, ld, w, col0, flag);
+    nopiv_diag_steps<CPLX, 12>(v, scol, srow, a, ld, w, col0, flag);
+    nopiv_diag_steps<CPLX, 8>(v, scol, srow, a, ld, w, col0, flag);
+    nopiv_diag_steps<CPLX, 4>(v, scol, srow, a, ld, w, col0, flag);
 }
 
 // X := X U^-1 for the rows x w block X (w <= 64) and the w x w upper factor
-// U (staged in shared memory): one warp per row, lane l holding columns l and
-// l + 32; step k divides x_k by u_kk in its lane, broadcasts it, and the lanes
-// of the columns beyond k subtract x_k u_kc.
-template <bool CPLX>
-__global__ void __launch_bounds__(256) trsm_right_upper_kernel(const double* u, int ldu, double* x, int ldx,
-                                                             int rows, int w) {
-    constexpr int ES = CPLX ? 2 : 1;
-    extern __shared__ __align__(16) unsigned char nopiv_smem[];
-    Z* su = reinterpret_cast<Z*>(nopiv_smem);  // su[c * kNopivLd + r]
-    stage_block<CPLX>(su, u, ldu, w, w, true);
-    __syncthreads();
-    const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
-    for (int row = blockIdx.x * warps + (threadIdx.x >> 5); row < rows; row += gridDim.x * warps) {
-        Z v[2];
+// U (staged in shared memory): LN lanes per row, lane l holding columns l,
+// l + LN, ...; step k divides x_k by u_kk (by a reciprocal prepared for all
+// rows, correctly rounded), broadcasts it, and the columns beyond k subtract
+// x_k u_kc. Finished columns leave the first register as in the kernel above.
+// Bound by the steps' latency: 23 us for up to 4032 rows of 64 (a warp per row,
+// two columns a lane and a full division per step: 35).
+constexpr int kRightRows = 128;  // threads per CTA
+template <bool CPLX, int NQ, int LN>
+__device__ __forceinline__ void right_upper_steps(Z (&v)[kNopivBlock / LN], const Z* su, const Divisor* sdiv, int ln,
+                                                  bool live, double* x, int ldx, int row, int w) {
+    constexpr int ES = CPLX ? 2 : 1, Q = kNopivBlock / LN;
+    using E = std::conditional_t<CPLX, double2, double>;
+    for (int q0 = Q - NQ; q0 < Q - NQ + Q / 4 && LN * q0 < w; ++q0) {
 #pragma unroll
-        for (int q = 0; q < 2; ++q) {
-            const int c = lane + 32 * q;
-            v[q] = c < w ? load_el<CPLX>(x + ((size_t)c * ldx + row) * ES) : Z{0.0, 0.0};
-        }
-        for (int k = 0; k < w; ++k) {
-            const int h = k >> 5, src = k & 31;
-            if (lane == src) v[h] = div_el<CPLX>(v[h], su[k * kNopivLd + k]);
-            const Z xk{__shfl_sync(0xffffffffu, v[h].re, src), CPLX ? __shfl_sync(0xffffffffu, v[h].im, src) : 0.0};
+        for (int i = 0; i < LN; ++i) {
+            const int k = LN * q0 + i;
+            const Divisor d = sdiv[k];
+            Z u[NQ];
 #pragma unroll
-            for (int q = 0; q < 2; ++q) {
-                const int c = lane + 32 * q;
-                if (c > k && c < w) v[q] = sub_prod<CPLX>(v[q], xk, su[c * kNopivLd + k]);
+            for (int q = 0; q < NQ; ++q) u[q] = su[(LN * (q0 + q < Q ? q0 + q : q0) + ln) * kNopivLd + k];
+            E num, y;
+            if constexpr (CPLX) num = make_double2(v[0].re, v[0].im);
+            else num = v[0].re;
+            const bool fast = divide_fast(num, d, y);
+            if (ln == i && !(fast && d.safe)) y = divide(num, d);
+            Z xk{0.0, 0.0};
+            if constexpr (CPLX) {
+                xk.re = __shfl_sync(0xffffffffu, y.x, i, LN);
+                xk.im = __shfl_sync(0xffffffffu, y.y, i, LN);
+            } else {
+                xk.re = __shfl_sync(0xffffffffu, y, i, LN);
             }
-        }
 #pragma unroll
-        for (int q = 0; q < 2; ++q) {
-            const int c = lane + 32 * q;
-            if (c < w) store_el<CPLX>(x + ((size_t)c * ldx + row) * ES, v[q]);
+            for (int q = 0; q < NQ; ++q) {
+                const Z t = sub_prod<CPLX>(v[q], xk, u[q]);
+                const bool take = q > 0 || ln > i;
+                v[q].re = take ? t.re : v[q].re;
+                if (CPLX) v[q].im = take ? t.im : v[q].im;
+            }
+            v[0].re = ln == i ? xk.re : v[0].re;
+            if (CPLX) v[0].im = ln == i ? xk.im : v[0].im;
         }
+        const int c = LN * q0 + ln;
+        if (live && c < w) store_el<CPLX>(x + ((size_t)c * ldx + row) * ES, v[0]);
+#pragma unroll
+        for (int q = 0; q + 1 < NQ; ++q) v[q] = v[q + 1];
     }
 }
 
-constexpr int kNopivDiagSmem = kNopivBlock * kNopivLd * 16;
+template <bool CPLX>
+__global__ void __launch_bounds__(kRightRows) trsm_right_upper_kernel(const double* u, int ldu, double* x, int ldx,
+                                                                    int rows, int w) {
+    constexpr int ES = CPLX ? 2 : 1, LN = CPLX ? 8 : 4, Q = kNopivBlock / LN;
+    extern __shared__ __align__(16) unsigned char nopiv_smem[];
+    Z* su = reinterpret_cast<Z*>(nopiv_smem);  // su[c * kNopivLd + r]
+    __shared__ Divisor sdiv[kNopivBlock];
+    stage_block<CPLX>(su, u, ldu, w, w, true);
+    __syncthreads();
+    if (threadIdx.x < kNopivBlock) {
+        const Z d = (int)threadIdx.x < w ? su[threadIdx.x * kNopivLd + threadIdx.x] : Z{1.0, 0.0};
+        if constexpr (CPLX) sdiv[threadIdx.x] = make_divisor(make_double2(d.re, d.im));
+        else sdiv[threadIdx.x] = make_divisor(d.re);
+    }
+    __syncthreads();
+    const int ln = threadIdx.x % LN, row = (blockIdx.x * kRightRows + threadIdx.x) / LN;
+    Z v[Q];
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+        const int c = LN * q + ln;
+        v[q] = row < rows && c < w ? load_el<CPLX>(x + ((size_t)c * ldx + row) * ES) : Z{0.0, 0.0};
+    }
+    right_upper_steps<CPLX, Q, LN>(v, su, sdiv, ln, row < rows, x, ldx, row, w);
+    right_upper_steps<CPLX, Q * 3 / 4, LN>(v, su, sdiv, ln, row < rows, x, ldx, row, w);
+    right_upper_steps<CPLX, Q / 2, LN>(v, su, sdiv, ln, row < rows, x, ldx, row, w);
+    right_upper_steps<CPLX, Q / 4, LN>(v, su, sdiv, ln, row < rows, x, ldx, row, w);
+}
+
 constexpr int kNopivTrsmSmem = kNopivBlock * kNopivLd * 16;
 
 template <bool CPLX>
@@ -2239,8 +2340,6 @@ void configure_nopiv_kernels() {
     int dev = 0;
     TNS_CUDA(cudaGetDevice(&dev));
     if (dev >= 0 && dev < 64 && done[dev]) return;
-    TNS_CUDA(cudaFuncSetAttribute(lu_nopiv_diag_kernel<CPLX>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  kNopivDiagSmem));
     TNS_CUDA(cudaFuncSetAttribute(trsm_right_upper_kernel<CPLX>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   kNopivTrsmSmem));
     if (dev >= 0 && dev < 64) done[dev] = true;
@@ -2488,25 +2587,25 @@ void lu_nopiv_panel(Context& ctx, DMat& a, int j, int w, int* flag) {
     else configure_nopiv_kernels<false>();
     for (int b0 = 0; b0 < w; b0 += kNopivBlock) {
         const int bw = std::min(kNopivBlock, w - b0), k = j + b0;
-        if (cplx) lu_nopiv_diag_kernel<true><<<1, 256, kNopivDiagSmem, ctx.stream>>>(a.at(k, k), ld, bw, k, flag);
-        else lu_nopiv_diag_kernel<false><<<1, 256, kNopivDiagSmem, ctx.stream>>>(a.at(k, k), ld, bw, k, flag);
+        if (cplx) lu_nopiv_diag_kernel<true><<<1, 256, 0, ctx.stream>>>(a.at(k, k), ld, bw, k, flag);
+        else lu_nopiv_diag_kernel<false><<<1, 256, 0, ctx.stream>>>(a.at(k, k), ld, bw, k, flag);
         TNS_CUDA(cudaGetLastError());
         ctx.kernel_launches++;
         const int below = n - k - bw, right = w - b0 - bw;
         if (below > 0) {
-            const int grid = std::min((below + 7) / 8, ctx.num_sms * 2);
+            const int per_cta = kRightRows / (cplx ? 8 : 4), grid = (below + per_cta - 1) / per_cta;
             if (cplx)
-                trsm_right_upper_kernel<true><<<grid, 256, kNopivTrsmSmem, ctx.stream>>>(a.at(k, k), ld,
+                trsm_right_upper_kernel<true><<<grid, kRightRows, kNopivTrsmSmem, ctx.stream>>>(a.at(k, k), ld,
                                                                                         a.at(k + bw, k), ld, below, bw);
             else
-                trsm_right_upper_kernel<false><<<grid, 256, kNopivTrsmSmem, ctx.stream>>>(a.at(k, k), ld,
+                trsm_right_upper_kernel<false><<<grid, kRightRows, kNopivTrsmSmem, ctx.stream>>>(a.at(k, k), ld,
                                                                                          a.at(k + bw, k), ld, below, bw);
             TNS_CUDA(cudaGetLastError());
             ctx.kernel_launches++;
         }
         if (right > 0) {
-            std::vector<TrsmDesc> t{TrsmDesc{a.at(k, k), ld, a.at(k, k + bw), ld, bw, right, 1, 1, 0}};
-            launch_trsm(ctx, cplx, t);
+            std::vector<PanelRowsDesc> u{PanelRowsDesc{a.p, ld, k + bw, k + bw + right, nullptr, k, bw, 0, 1, 0}};
+            launch_panel_rows(ctx, cplx, u);
             if (below > 0) {
                 GemmProblem p{};
                 p.A = a.at(k + bw, k);
@@ -2604,9 +2703,15 @@ bool gesv_mixed_butterfly(Context& ctx, const DMat& a, const DMat& b, DMat& x, i
         return zero_at == INT_MAX;
     };
     // (LU)^-1 or (LU)^-H in place: a few columns (the estimator's probes)
-    // through the chained solve, wide panels by blocked TRSM + DMMA updates.
+    // through the chained solve, more through the one-launch solve (its
+    // interchanges the identity), many by blocked TRSM + DMMA updates.
+    DBuf identity(ctx, sizeof(int) * (size_t)N);
+    std::vector<int> order(N);
+    for (int i = 0; i < N; ++i) order[i] = i;
+    TNS_CUDA(cudaMemcpyAsync(identity.p, order.data(), sizeof(int) * N, cudaMemcpyHostToDevice, ctx.stream));
     auto lu_solve = [&](DMat& m, int cols, bool adjoint) {
         if (cols <= 2 * kChainCols) chain_solve(ctx, f, inverses.as<double>(), m, cols, adjoint);
+        else if (cols <= kOneLaunchCols && !adjoint) getrs(ctx, f, identity.as<int>(), m, cols, false);
         else getrs_free_order(ctx, f, nullptr, m, cols, adjoint);
     };
     // M := A^-1 M or A^-H M in place on an N-row panel (zeros below row n).
