@@ -86,6 +86,30 @@ DMat upload(Context& ctx, const double* src, int rows, int cols, int ld, bool cp
     return m;
 }
 
+// A product's A or B where it lies, when the kernel can read it there: device
+// memory of this device, even rows and whole 16-deep k steps (what its loops
+// run over without padding), and the 16-byte alignment of TMA's base and
+// strides. Otherwise (null) it is copied into a padded matrix. 1024^3 in place
+// 138 us, copied 171 (two allocations, two clears, two copies of 8 MB).
+DMat in_place(Context& ctx, const double* p, int rows, int cols, int ld, bool cplx, bool fits, const char* purpose) {
+    DMat m;
+    const size_t esz = cplx ? 16 : 8;
+    cudaPointerAttributes at{};
+    if (!fits || reinterpret_cast<uintptr_t>(p) % 16 || (size_t)ld * esz % 16) return m;
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        cudaGetLastError();
+        return m;
+    }
+    if (at.type != cudaMemoryTypeDevice || at.device != ctx.device) return m;
+    ctx.check_limit((long long)rows * cols, purpose);
+    m.p = const_cast<double*>(p);  // not owned: no context
+    m.rows = rows;
+    m.cols = m.cols_p = cols;
+    m.rows_p = ld;
+    m.cplx = cplx;
+    return m;
+}
+
 int gemm_entry(tns_context* c, bool cplx, bool dev, int m, int n, int k, const double* alpha, const double* a, int lda,
                const double* b, int ldb, const double* beta, double* cm, int ldc) {
     return guarded(c, [&](Context& ctx) {
@@ -94,8 +118,11 @@ int gemm_entry(tns_context* c, bool cplx, bool dev, int m, int n, int k, const d
         check_operand(b, k, n, ldb, "B");
         check_operand(cm, m, n, ldc, "C");
         if (m == 0 || n == 0) return;
-        DMat A = upload(ctx, a, m, k, lda, cplx, dev, "the A operand");
-        DMat B = upload(ctx, b, k, n, ldb, cplx, dev, "the B operand");
+        const bool whole = dev && k > 0 && k % 16 == 0;
+        DMat A = in_place(ctx, a, m, k, lda, cplx, whole && m % 2 == 0, "the A operand");
+        if (!A.p) A = upload(ctx, a, m, k, lda, cplx, dev, "the A operand");
+        DMat B = in_place(ctx, b, k, n, ldb, cplx, whole && n % 2 == 0, "the B operand");
+        if (!B.p) B = upload(ctx, b, k, n, ldb, cplx, dev, "the B operand");
         bool need_c = !(beta[0] == 0.0 && beta[1] == 0.0);
         DMat C = need_c ? upload(ctx, cm, m, n, ldc, cplx, dev, "the C operand") : DMat(ctx, m, n, cplx, "the C operand");
         if (!cplx && alpha[0] == 0.0) {

@@ -4,7 +4,8 @@
 // Right-looking blocked getrf as the reference runs it (src/Tensile.Kernels/Lu.cs:230-309
 // for real, src/Tensile/BlockedLu.cs:45-101 for complex): per block of nb
 // columns
-//   1. panel factorization (one CTA per matrix; pivot = first index of the
+//   1. panel factorization (a cluster per matrix, lu_panel.cu, where the rows
+//      fit its registers, else one CTA or all SMs; pivot = first index of the
 //      largest |a|, or |Re|+|Im| for complex; reciprocal multiply unless
 //      |pivot| < SafeMin; rank-1 updates y + (-m)*x with two roundings),
 //   2. the panel's row interchanges applied to the columns either side, and
@@ -17,8 +18,8 @@
 // launch per phase (a grouped GEMM for the trailing updates).
 //
 // Solves: forward and backward substitution in the reference's order, blocked
-// into 32-row diagonal solves and register-tiled updates that continue each
-// element's chain of roundings in the reference's order, so A^-1 B -- the Pade
+// into diagonal solves and register-tiled updates (one launch for a single
+// system, subst_cols.cu) that continue each element's chain of roundings in the reference's order, so A^-1 B -- the Pade
 // solve included -- matches the reference bit for bit. The adjoint solves,
 // whose reference order is an inner product per row, run left-looking: ColumnOps.Dot's
 // vector order for real factors, sequential sums for complex ones (the forward
