@@ -1099,7 +1099,10 @@ void expmv_batch(Context& ctx, const std::vector<const DMat*>& as, const std::ve
     L.ncols = ncols;
     L.err = ctx.d_err;
     L.progress = state.as<unsigned long long>();
-    L.maps = static_cast<const CUtensorMap*>(ctx.upload(maps.data(), sizeof(CUtensorMap) * cnt));
+    // (A buffer of their own: beside the descriptors they could outgrow the upload ring.)
+    DBuf dmaps(ctx, sizeof(CUtensorMap) * cnt);
+    TNS_CUDA(cudaMemcpyAsync(dmaps.p, maps.data(), sizeof(CUtensorMap) * cnt, cudaMemcpyHostToDevice, ctx.stream));
+    L.maps = dmaps.as<CUtensorMap>();
     taylor(ctx, cplx, skip, ncols, &L, lay.lanes);
     std::vector<int> h(2 * cnt);
     TNS_CUDA(cudaMemcpyAsync(h.data(), outs, sizeof(int) * 2 * cnt, cudaMemcpyDeviceToHost, ctx.stream));
