@@ -420,6 +420,9 @@ __global__ void __launch_bounds__(kMaxThreads<CPLX>, 1)
         if (ok && s.limit > 8) ok = panel_phase<CPLX, 24>(s, a, pos, 8);
         if (ok && s.limit > 16) ok = panel_phase<CPLX, 16>(s, a, pos, 16);
         if (ok && s.limit > 24) ok = panel_phase<CPLX, 8>(s, a, pos, 24);
+        // A pivot row's entries were stored by the lanes of its warp; after the
+        // last column no block barrier lies between that and reading them here.
+        __syncwarp();
         if (ok && row < M) {
             for (int c = 0; c < d.w; ++c) P[(size_t)c * d.ld + pos] = s.save[(size_t)c * T];
             if (d.carry > 0 && pos != row) {

@@ -1,0 +1,23 @@
+"""Values that the lanes of a warp hand to one another through shared memory,
+each lane's in turn, bit for bit against the oracle."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("m,n", [(1, 32), (5, 32), (20, 60), (31, 32), (32, 32), (40, 64)])
+@pytest.mark.parametrize("cplx", [False, True])
+def test_last_pivot_row_from_every_lane(ws, orc, m, n, cplx):
+    """Panels of no more rows than columns, whose last pivot row, of several
+    entries, is each row in turn: its lane stores what the others hold."""
+    rng = np.random.default_rng(m + n)
+    base = rng.uniform(-0.1, 0.1, (m, n)) + (1j * rng.uniform(-0.1, 0.1, (m, n)) if cplx else 0)
+    base[np.arange(m), np.arange(m)] += 4.0
+    for last in range(m):
+        order = np.delete(np.arange(m - 1, -1, -1), 0)  # the other pivots, in reverse
+        a = base[np.insert(order, last, m - 1)]
+        lu = ws.factor_lu(a, 64)
+        f, piv, _ = orc.getrf(a, 64)
+        assert np.array_equal(lu.pivots, piv)
+        assert np.array_equal(lu.factors, f)
