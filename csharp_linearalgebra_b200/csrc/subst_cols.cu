@@ -251,6 +251,7 @@ __device__ __forceinline__ void triangle(const typename El<CPLX>::T* t, int w, t
         mine.safe = 1;
         if (lane < w) mine = make_divisor(t[lane * kB + lane]);
         dv[lane] = mine;
+        __syncwarp();  // a vote orders no memory
         const bool all_safe = __all_sync(0xffffffffu, mine.safe);
         E kept[NQ];
 #pragma unroll

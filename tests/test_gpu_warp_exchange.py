@@ -21,3 +21,22 @@ def test_last_pivot_row_from_every_lane(ws, orc, m, n, cplx):
         f, piv, _ = orc.getrf(a, 64)
         assert np.array_equal(lu.pivots, piv)
         assert np.array_equal(lu.factors, f)
+
+
+@pytest.mark.parametrize("n", [1, 2, 31, 32, 33, 100])
+@pytest.mark.parametrize("cplx", [False, True])
+def test_divisors_from_every_lane(ws, orc, n, cplx):
+    """Triangles whose diagonal differs in every row: each lane prepares one
+    divisor, and every lane divides by all of them in turn."""
+    rng = np.random.default_rng(n)
+
+    def part(*shape):
+        return rng.uniform(-1.0, 1.0, shape)
+
+    a = part(n, n) / n + (1j * part(n, n) / n if cplx else 0)
+    a[np.arange(n), np.arange(n)] = (1.0 + rng.uniform(size=n)) * 3.0 ** rng.integers(-9, 10, n) * \
+        (np.exp(2j * np.pi * rng.uniform(size=n)) if cplx else rng.choice([-1.0, 1.0], n))
+    for nrhs in (1, 4, 40, 500):  # one column a CTA, and several
+        b = part(n, nrhs) + (1j * part(n, nrhs) if cplx else 0)
+        for tri in ("upper",) + (() if cplx else ("lower",)):
+            assert np.array_equal(ws.solve_triangular(tri, a, b), orc.trsolve(tri, a, b)), (tri, nrhs)
