@@ -845,11 +845,15 @@ __global__ void build_perm_kernel(const __grid_constant__ Batch<PermDesc> b) {
     for (int i = threadIdx.x; i < n; i += blockDim.x) root[i] = last[i] < 0 ? i : last[i];
     __syncthreads();
     for (;;) {
+        // Each thread advances its own entries while others read them: an
+        // ancestor either way, so concurrent steps only shorten the way. The
+        // accesses are volatile, so that each is one access of a whole word.
+        volatile int* way = root;
         int changed = 0;
         for (int i = threadIdx.x; i < n; i += blockDim.x) {
-            const int r = root[i], rr = root[r];
+            const int r = way[i], rr = way[r];
             if (rr != r) {
-                root[i] = rr;  // an ancestor either way: concurrent steps only shorten the way
+                way[i] = rr;
                 changed = 1;
             }
         }

@@ -40,3 +40,21 @@ def test_divisors_from_every_lane(ws, orc, n, cplx):
         b = part(n, nrhs) + (1j * part(n, nrhs) if cplx else 0)
         for tri in ("upper",) + (() if cplx else ("lower",)):
             assert np.array_equal(ws.solve_triangular(tri, a, b), orc.trsolve(tri, a, b)), (tri, nrhs)
+
+
+@pytest.mark.parametrize("n", [1, 33, 257, 1500])
+@pytest.mark.parametrize("adjoint", [False, True])
+def test_long_chains_of_interchanges(ws, orc, n, adjoint):
+    """Pivot sequences whose interchanges pass a row along through hundreds of
+    others (each with the next row, or all with the last), which the threads
+    follow side by side."""
+    k = np.arange(n)
+    rng = np.random.default_rng(n)
+    f = np.eye(n) * 2.0 + rng.uniform(-0.5, 0.5, (n, n)) / n
+    b = rng.uniform(-1.0, 1.0, (n, 2))
+    for piv in (np.minimum(k + 1, n - 1), np.full(n, n - 1), np.maximum(k, n - 1 - k), rng.integers(k, n)):
+        x = np.asfortranarray(b.copy())
+        piv = piv.astype(np.int32)
+        ff = np.asfortranarray(f)
+        ws._call("tns_dgetrs", n, 2, ff.ctypes.data, n, piv.ctypes.data, -1, x.ctypes.data, n, int(adjoint))
+        assert np.array_equal(x, orc.getrs(f, piv, b, adjoint=adjoint))
