@@ -78,6 +78,7 @@ Context::~Context() {
     for (auto e : event_pool) cudaEventDestroy(e);
     copier.reset();
     if (split_scratch) cudaFree(split_scratch);
+    free_old_rings();
     if (h_ring) cudaFreeHost(h_ring);
     if (d_ring) cudaFree(d_ring);
     if (d_err) cudaFree(d_err);
@@ -94,23 +95,42 @@ cudaStream_t Context::copies() {
     return copy_stream;
 }
 
-const void* Context::upload(const void* src, size_t bytes) {
-    size_t need = (bytes + 255) & ~size_t(255);
-    if (need > ring_cap) {
-        // Grow: everything already queued must finish with the old ring.
-        TNS_CUDA(cudaStreamSynchronize(stream));
-        if (h_ring) TNS_CUDA(cudaFreeHost(h_ring));
-        if (d_ring) TNS_CUDA(cudaFree(d_ring));
-        h_ring = nullptr;
-        d_ring = nullptr;
-        ring_cap = std::max(need, size_t(4) << 20);
-        TNS_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&h_ring), ring_cap, cudaHostAllocDefault));
-        TNS_CUDA(cudaMalloc(reinterpret_cast<void**>(&d_ring), ring_cap));
-        ring_pos = 0;
+void Context::free_old_rings() {
+    for (auto& r : old_rings) {
+        cudaFreeHost(r.first);
+        cudaFree(r.second);
     }
-    if (ring_pos + need > ring_cap) {
-        // Wrap around: the copies and kernels still reading the ring finish first.
+    old_rings.clear();
+}
+
+const void* Context::upload(const void* src, size_t bytes) {
+    const size_t need = (bytes + 255) & ~size_t(255);
+    if (ring_pos + need > (ring_held && hold_wrapped ? hold_from : ring_cap)) {
+        // The copies and kernels still reading the ring finish first.
         TNS_CUDA(cudaStreamSynchronize(stream));
+        if (!ring_held) free_old_rings();
+        // Wrap around, where a hold's own uploads leave room for it, or grow.
+        if (need <= (!ring_held ? ring_cap : hold_wrapped ? 0 : hold_from)) {
+            hold_wrapped = ring_held;
+        } else {
+            const size_t cap = std::max({need, size_t(4) << 20, ring_held ? 2 * ring_cap : size_t(0)});
+            if (h_ring) {
+                old_rings.emplace_back(h_ring, d_ring);
+                h_ring = d_ring = nullptr;
+                ring_cap = 0;
+            }
+            if (!ring_held) free_old_rings();
+            char *host = nullptr, *dev = nullptr;
+            TNS_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&host), cap, cudaHostAllocDefault));
+            const cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&dev), cap);
+            if (e != cudaSuccess) cudaFreeHost(host);
+            TNS_CUDA(e);
+            h_ring = host;
+            d_ring = dev;
+            ring_cap = cap;
+            hold_from = 0;
+            hold_wrapped = false;
+        }
         ring_pos = 0;
     }
     std::memcpy(h_ring + ring_pos, src, bytes);

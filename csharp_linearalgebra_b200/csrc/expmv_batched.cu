@@ -1093,6 +1093,7 @@ void expmv_batch(Context& ctx, const std::vector<const DMat*>& as, const std::ve
         d.eta_one = (eta_re[k] == 1.0 && eta_im[k] == 0.0) ? 1 : 0;
     }
     TaylorLaunch L{};
+    UploadHold hold(ctx);  // the descriptors, the plan and its offsets
     L.descs = static_cast<const TaylorDesc*>(ctx.upload(descs.data(), sizeof(TaylorDesc) * cnt));
     L.plan = static_cast<const TaylorPlan*>(ctx.upload(sc.plan.data(), sizeof(TaylorPlan) * std::max<size_t>(sc.plan.size(), 1)));
     L.plan_off = static_cast<const int*>(ctx.upload(sc.offsets.data(), sizeof(int) * sc.offsets.size()));

@@ -669,6 +669,7 @@ void launch_cfg(Context& ctx, std::vector<GemmProblem>& probs, const std::functi
     L.err = ctx.d_err;
     L.tiles = ctx.d_tiles;
     TNS_CUDA(cudaMemsetAsync(ctx.d_tiles, 0, sizeof(unsigned long long), ctx.stream));
+    UploadHold hold(ctx);  // the problems and their maps
     if (probs.size() <= 4) {
         for (size_t i = 0; i < probs.size(); ++i) {
             L.inl[i] = probs[i];

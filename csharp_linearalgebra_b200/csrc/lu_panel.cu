@@ -466,6 +466,7 @@ void launch(Context& ctx, const std::vector<PanelFactorDesc>& v) {
     const int cs = std::max(1, (rows_max + top - 1) / top);
     const int threads = round_up((rows_max + cs - 1) / cs, 32);
     if (cs > kMaxCluster) fail(TNS_E_ARGUMENT, "internal: panel too tall for the register kernel");
+    UploadHold hold(ctx);  // the slots and the panels
     const PanelSlot* d_slots = nullptr;
     int grid = cs;
     if (v.size() > 1) {

@@ -1170,6 +1170,7 @@ void split_launch(Context& ctx, std::vector<SplitProduct>& v, int nm) {
         TNS_CUDA(cudaGetLastError());
         ctx.kernel_launches += 4;
     }
+    UploadHold hold(ctx);  // descriptors and maps, of up to two launches
     const ModDesc* d_desc = static_cast<const ModDesc*>(ctx.upload(md.data(), sizeof(ModDesc) * md.size()));
     const ModMaps* d_maps = static_cast<const ModMaps*>(ctx.upload(maps.data(), sizeof(ModMaps) * maps.size()));
     cudaEvent_t e0 = nullptr, e1 = nullptr;

@@ -85,11 +85,20 @@ struct Context {
     long long kernel_launches = 0;  // kernels launched through this context
     // Launch descriptors go to the device through a ring of pinned host memory
     // mirrored in device memory, so that uploading them never blocks the host
-    // on the stream. Wrapping around synchronises the stream once.
+    // on the stream. Wrapping around synchronises the stream once. An upload is
+    // good for the launches queued before the next one; several for one launch
+    // are made under an UploadHold.
     char* h_ring = nullptr;
     char* d_ring = nullptr;
     size_t ring_cap = 0, ring_pos = 0;
     const void* upload(const void* src, size_t bytes);
+    // Of the hold in force: where its uploads start in the ring, and whether
+    // they go on at its beginning.
+    bool ring_held = false, hold_wrapped = false;
+    size_t hold_from = 0;
+    // Rings that were outgrown under a hold, kept for the launch they belong to.
+    std::vector<std::pair<char*, char*>> old_rings;  // host, device
+    void free_old_rings();
 
     // Optional per-launch timing of the GEMM kernel (CUDA events on this
     // context's stream), for the roofline report.
@@ -163,6 +172,26 @@ struct Context {
     ~Context();
     void sync();                       // stream sync + device error flag check
     void check_limit(long long elements, const char* purpose) const;
+};
+
+// The uploads made while one is in force stay where they are until it ends: a
+// launch that takes several of them is queued before that. (Without it, the
+// second upload may take the place of the first, by wrapping around the ring,
+// or give the first one's memory back, by outgrowing it.)
+struct UploadHold {
+    Context& ctx;
+    const bool outer;
+    explicit UploadHold(Context& c) : ctx(c), outer(c.ring_held) {
+        if (outer) return;
+        ctx.ring_held = true;
+        ctx.hold_wrapped = false;
+        ctx.hold_from = ctx.ring_pos;
+    }
+    ~UploadHold() {
+        if (!outer) ctx.ring_held = false;
+    }
+    UploadHold(const UploadHold&) = delete;
+    UploadHold& operator=(const UploadHold&) = delete;
 };
 
 // A padded device matrix owned by the library: rows_p x cols_p with
