@@ -5,7 +5,7 @@
 #include <algorithm>
 #include <cstdint>
 #include <cstring>
-#include <system_error>
+#include <exception>
 #if defined(__SSE2__)
 #include <emmintrin.h>
 #endif
@@ -30,9 +30,12 @@ HostCopier::HostCopier(int device) : device_(device) {
             }
         }
     try {
+        helpers_.reserve(threads - 1);
         for (int t = 1; t < threads; ++t) helpers_.emplace_back([this, t] { helper(t); });
-    } catch (const std::system_error&) {
-        // Fewer helpers then; the calling thread alone in the worst case.
+    } catch (const std::exception&) {
+        // No thread (system_error) or no memory for one (bad_alloc): fewer
+        // helpers then, the calling thread alone in the worst case. Nothing may
+        // leave here, since the destructor that joins them would not run.
     }
 }
 
