@@ -140,8 +140,8 @@ struct Pieces {
         cols_per = std::max<size_t>(1, HostCopier::kPiece / column);
         // At least four pieces, so that packing and the bus overlap.
         cols_per = std::min(cols_per, std::max<size_t>(1, (cols + 3) / 4));
-        parts = (column + HostCopier::kPiece - 1) / HostCopier::kPiece;
-        part = HostCopier::kPiece;
+        part = std::clamp(column * cols / 4, HostCopier::kLeast, HostCopier::kPiece);
+        parts = (column + part - 1) / part;
         count = parts > 1 ? cols * parts : (cols + cols_per - 1) / cols_per;
     }
     // Piece i: `bytes` of the padded side from `offset` on.
