@@ -773,7 +773,8 @@ bool slab_split_launch(Context& ctx, const std::vector<GemmProblem>& work, long 
     return true;
 }
 
-void gemm_run(Context& ctx, std::vector<GemmProblem>& probs, bool cplx) {
+// single: a public call's product, which is split wherever that applies.
+void gemm_run(Context& ctx, std::vector<GemmProblem>& probs, bool cplx, bool single) {
     std::vector<GemmProblem> work;
     work.reserve(probs.size());
     for (auto& p0 : probs) {
@@ -802,8 +803,10 @@ void gemm_run(Context& ctx, std::vector<GemmProblem>& probs, bool cplx) {
         depth = std::max(depth, p.K);
         if (p.beta_re != 0.0 || p.beta_im != 0.0) overwrite = false;
     }
-    // Not in a batch worker: the other workers' launches fill the idle SMs.
-    if (!ctx.concurrent && work.size() <= kSlabSplitProblems &&
+    // Not in a batch worker: the other workers' launches fill the idle SMs. Nor
+    // inside an algorithm when the autotuner is to choose the shape: it times
+    // the unsplit kernel's two.
+    if (!ctx.concurrent && (single || !ctx.autotune) && work.size() <= kSlabSplitProblems &&
         (cplx ? slab_split_launch<CplxBig, CplxSmall>(ctx, work, tiles)
               : slab_split_launch<RealBig, RealSmall>(ctx, work, tiles)))
         return;
@@ -840,11 +843,11 @@ void gemm_run(Context& ctx, std::vector<GemmProblem>& probs, bool cplx) {
 
 }  // namespace
 
-void gemm_grouped(Context& ctx, std::vector<GemmProblem>& probs, bool cplx) { gemm_run(ctx, probs, cplx); }
+void gemm_grouped(Context& ctx, std::vector<GemmProblem>& probs, bool cplx) { gemm_run(ctx, probs, cplx, false); }
 
 void gemm(Context& ctx, const GemmProblem& p, bool cplx) {
     std::vector<GemmProblem> v{p};
-    gemm_run(ctx, v, cplx);
+    gemm_run(ctx, v, cplx, true);
 }
 
 namespace {
