@@ -735,7 +735,7 @@ constexpr size_t kSlabSplitProblems = 4;
 // work at once, each unit's raw slab product goes to its own plane, and a fold
 // kernel adds the slabs into C in slab order with the operations the unsplit
 // kernel applies at each slab end (the same bits). False when the split does
-// not apply.
+// not apply or its planes are not to be had.
 template <class Big, class Small>
 bool slab_split_launch(Context& ctx, const std::vector<GemmProblem>& work, long long tiles_big) {
     constexpr bool CPLX = Big::kComplex;
@@ -751,7 +751,14 @@ bool slab_split_launch(Context& ctx, const std::vector<GemmProblem>& work, long 
         units_big += (long long)((p.M + Big::BM - 1) / Big::BM) * ((p.N + Big::BN - 1) / Big::BN) * slabs * passes;
     }
     if (most < 2 || bytes > kSlabPlaneBytes) return false;
-    DBuf planes(ctx, bytes);
+    DBuf planes;
+    try {
+        planes = DBuf(ctx, bytes);
+    } catch (const Error& e) {
+        // No memory for the planes, which the unsplit kernel does without.
+        if (e.code != TNS_E_OUT_OF_MEMORY) throw;
+        return false;
+    }
     std::vector<GemmProblem> v = work;
     size_t at = 0;
     for (auto& p : v) {

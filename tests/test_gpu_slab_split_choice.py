@@ -4,7 +4,10 @@ import os
 import subprocess
 import sys
 
+import numpy as np
 import pytest
+
+from csharp_linearalgebra_b200 import _native
 
 pytestmark = pytest.mark.gpu
 
@@ -36,3 +39,32 @@ with Workspace() as ws:
     r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300,
                        cwd=ROOT)
     assert r.returncode == 0, r.stderr
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+def test_without_memory_for_the_planes(ws, cplx):
+    """Every device allocation of an exponential refused in turn: the planes'
+    refusals cost nothing but the split, every other one is reported."""
+    rng = np.random.default_rng(2)
+    n = 384  # two slabs of 256, and no padding
+    a = rng.standard_normal((n, n)) + (1j * rng.standard_normal((n, n)) if cplx else 0)
+    a = np.asfortranarray(a * (20.0 / np.abs(a).sum(axis=0).max()))
+    want = ws.expm(a)
+    lib = _native.load()
+    reported = unsplit = 0
+    for k in range(1, 2000):
+        assert lib.tns_inject_allocation_failure(ws.handle, k) == 0
+        try:
+            got = ws.expm(a)
+        except MemoryError:
+            reported += 1
+            continue
+        assert np.array_equal(got, want)
+        try:
+            ws.multiply(np.eye(2), np.eye(2))  # a refusal that is still to come
+        except MemoryError:
+            break
+        unsplit += 1
+    else:
+        pytest.fail("no exponential went without a refusal")
+    assert reported > 20 and unsplit >= 6
