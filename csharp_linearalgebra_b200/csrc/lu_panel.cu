@@ -475,18 +475,22 @@ void launch(Context& ctx, const std::vector<PanelFactorDesc>& v) {
         std::iota(order.begin(), order.end(), 0);
         auto size_of = [&](int i) { return std::max(1, (v[i].m - v[i].r0 + threads - 1) / threads); };
         std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return size_of(x) > size_of(y); });
+        // Each into the fullest cluster that has room for it.
         std::vector<PanelSlot> slots;
-        std::vector<int> used;  // CTAs taken in each cluster
+        std::vector<int> open[kMaxCluster];  // clusters by their free CTAs
         for (int i : order) {
             const int g = size_of(i);
-            size_t k = 0;
-            while (k < used.size() && used[k] + g > cs) ++k;
-            if (k == used.size()) {
-                used.push_back(0);
+            int left = g;
+            while (left < cs && open[left].empty()) ++left;
+            size_t k = slots.size() / cs;
+            if (left < cs) {
+                k = open[left].back();
+                open[left].pop_back();
+            } else {
                 slots.resize(slots.size() + cs, PanelSlot{-1, 0, 0, 0});
             }
-            for (int r = 0; r < g; ++r) slots[k * cs + used[k] + r] = PanelSlot{i, r, g, used[k]};
-            used[k] += g;
+            for (int r = 0; r < g; ++r) slots[k * cs + cs - left + r] = PanelSlot{i, r, g, cs - left};
+            if (left > g) open[left - g].push_back((int)k);
         }
         grid = (int)slots.size();
         d_slots = static_cast<const PanelSlot*>(ctx.upload(slots.data(), sizeof(PanelSlot) * slots.size()));
