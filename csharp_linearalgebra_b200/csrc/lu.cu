@@ -1593,11 +1593,18 @@ void getrs_batch(Context& ctx, std::vector<SolveItem>& items, bool adjoint) {
         for (auto& it : items)
             all.push_back(SubstItem{it.lu->p, it.lu->ld(), it.b->p, it.b->ld(), it.lu->rows, it.nrhs});
         const bool wide = wide_batch(ctx, all);
-        for (auto& it : items) {
+        std::vector<SubstItem> subst;  // the items solved by blocks
+        for (size_t q = 0; q < items.size(); ++q) {
+            auto& it = items[q];
             int n = it.lu->rows;
             if (n == 0 || it.nrhs == 0) continue;
-            if (!wide && n <= kGatherMaxRows && n <= subst_cols_max_order(cplx)) fit.push_back(&it);
-            else if (it.nrhs < kGatherMaxCols && n <= kGatherMaxRows) narrow.push_back(&it);
+            const bool one_launch = !wide && n <= kGatherMaxRows && n <= subst_cols_max_order(cplx);
+            if (one_launch) {
+                fit.push_back(&it);
+                continue;
+            }
+            subst.push_back(all[q]);
+            if (it.nrhs < kGatherMaxCols && n <= kGatherMaxRows) narrow.push_back(&it);
             else swaps.push_back(LaswpDesc{it.b->p, it.b->ld(), 0, it.nrhs, it.d_piv, 0, n, 0});
         }
         if (!fit.empty()) {
@@ -1638,11 +1645,6 @@ void getrs_batch(Context& ctx, std::vector<SolveItem>& items, bool adjoint) {
                                          (size_t)narrow[q]->b->ld() * narrow[q]->nrhs * narrow[q]->b->esz(),
                                          cudaMemcpyDeviceToDevice, ctx.stream));
         }
-        std::vector<SubstItem> subst;
-        for (auto& it : items)
-            if (it.lu->rows > 0 && it.nrhs > 0 &&
-                std::none_of(fit.begin(), fit.end(), [&](const SolveItem* f) { return f == &it; }))
-                subst.push_back(SubstItem{it.lu->p, it.lu->ld(), it.b->p, it.b->ld(), it.lu->rows, it.nrhs});
         substitute(ctx, cplx, false, false, subst);  // L, unit diagonal, forward
         substitute(ctx, cplx, true, false, subst);   // U, backward
         return;
