@@ -1234,10 +1234,7 @@ __global__ void __launch_bounds__(64) left_subst_cplx_unit_back_kernel(const dou
 // step then reads nothing from global memory, and its sums are the kernels' above,
 // term for term. Complex: the products conj(f_ki) x[k] of a row are formed by
 // the half-warp, then one lane subtracts them in ascending k.
-constexpr int kStageSlots = 6;
 constexpr int kStageAhead = kStageSlots - 1;
-constexpr int kLeftRealMaxN = 3200;  // 6 slots + 2 columns of doubles: 200 KB
-constexpr int kLeftCplxMaxN = 1280;  // 6 slots + 2 columns + 2 product rows of complex: 200 KB
 
 template <bool FORWARD, bool UNIT>
 __global__ void __launch_bounds__(32) left_subst_real_staged_kernel(const double* __restrict__ f, int ldf, double* x,
@@ -1385,8 +1382,8 @@ void left_substitute(Context& ctx, bool cplx, bool forward, bool unit, const dou
         return;
     }
     const unsigned pairs = (unsigned)((nrhs + 1) / 2);
-    if (!cplx && n <= kLeftRealMaxN) {
-        const size_t smem = sizeof(double) * (size_t)(kStageSlots + 2) * n;
+    if (!cplx && n <= kStagedRealMaxN) {
+        const size_t smem = staged_left_smem(false, n);
         if (forward && !unit) {
             allow_left_smem<left_subst_real_staged_kernel<true, false>>(ctx.device);
             left_subst_real_staged_kernel<true, false><<<pairs, 32, smem, ctx.stream>>>(f, ldf, x, ldx, n, nrhs);
@@ -1401,8 +1398,8 @@ void left_substitute(Context& ctx, bool cplx, bool forward, bool unit, const dou
         ctx.kernel_launches++;
         return;
     }
-    if (cplx && !forward && unit && n <= kLeftCplxMaxN) {
-        const size_t smem = sizeof(double2) * (size_t)(kStageSlots + 4) * n;
+    if (cplx && !forward && unit && n <= kStagedCplxMaxN) {
+        const size_t smem = staged_left_smem(true, n);
         allow_left_smem<left_subst_cplx_unit_back_staged_kernel>(ctx.device);
         left_subst_cplx_unit_back_staged_kernel<<<pairs, 32, smem, ctx.stream>>>(f, ldf, x, ldx, n, nrhs);
         TNS_CUDA(cudaGetLastError());

@@ -433,12 +433,26 @@ bool left_solve_takes(const Context& ctx, bool cplx, int n, int nrhs) {
     if (!cplx && smem > kMaxSmem) smem = real_smem(n, 4) + kRealStatic;
     if (!cplx && smem > kMaxSmem) smem = real_smem(n, 2) + kRealStatic;
     if (smem > kMaxSmem) return false;
-    // CTAs at once, and so rounds of them. Against the staged kernels, which hold
-    // a thousand right-hand sides at once, a round takes a third of the time
-    // real (n = 512: 293 us against 877) and over half of it complex (n = 389:
-    // 442 us against 792).
-    const long long at_once = (long long)ctx.num_sms * std::max<size_t>(1, kMaxSmem / smem);
-    return nrhs <= at_once * (cplx ? 1 : 3);
+    // Each SM works on its right-hand sides as fast alone as together (real n =
+    // 256: 0.22 ms with one each, 0.36 with two, 0.49 with three), so the time
+    // goes by their rounds over the SMs; that of the staged kernels by the rounds
+    // of what their shared memory holds at once, a pair to a CTA. Measured over n
+    // = 32 .. 2700 real and 32 .. 1250 complex with up to 10,000 right-hand sides,
+    // the staged kernels' round takes as long as these of the new (ms, real:
+    // n = 64, 444: 0.17 against 0.20, 592: 0.21, 0.20; n = 512, 592: 1.31, 1.41,
+    // 740: 1.60, 1.44; n = 2048, 3000: 41, 67; complex n = 256, 1500: 1.30, 1.53,
+    // 6000: 4.3, 3.9; n = 1024, 1500: 31.2, 32.4, 6000: 115, 110).
+    auto rounds = [&](long long at_once) { return (nrhs + at_once - 1) / at_once; };
+    const double ours = (double)rounds(ctx.num_sms);
+    if (n > (cplx ? kStagedCplxMaxN : kStagedRealMaxN)) {
+        // The unstaged kernels, whose time hardly depends on their number (real n =
+        // 4096, 16 right-hand sides: 11 against 184 ms, 2000: 134, 195, 3000: 199,
+        // 202; complex n = 1400, 3000: 108, 134).
+        return ours <= (cplx ? 25 : 20);
+    }
+    const long long ctas = std::clamp<long long>(kMaxSmem / staged_left_smem(cplx, n), 1, 32);
+    const double per_round = cplx ? std::min(30.0, n < 900 ? 2048.0 / n : 1.85) : n > 64 ? 4.0 : 3.0;
+    return ours <= per_round * (double)rounds(2 * ctas * ctx.num_sms);
 }
 
 namespace {

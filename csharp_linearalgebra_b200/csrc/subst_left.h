@@ -18,9 +18,16 @@ struct LeftSolve {
     const int* perm;
 };
 
+// lu.cu's staged kernels, a warp per two right-hand sides with the factor's
+// columns in a ring of kStageSlots: the orders that fit their shared memory.
+constexpr int kStageSlots = 6;
+constexpr int kStagedRealMaxN = 3200;  // 6 slots + 2 columns of doubles: 200 KB
+constexpr int kStagedCplxMaxN = 1280;  // 6 slots + 2 columns + 2 product rows of complex: 200 KB
+inline size_t staged_left_smem(bool cplx, int n) { return (size_t)(cplx ? 16 * (kStageSlots + 4) : 8 * (kStageSlots + 2)) * n; }
+
 // Whether the kernels take a solve: its order's products fit shared memory, and
 // its right-hand sides, a CTA each, do not wait for one another so long that
-// the staged kernels of lu.cu (a warp per two right-hand sides) end first.
+// the kernels of lu.cu end first.
 bool left_solve_takes(const Context& ctx, bool cplx, int n, int nrhs);
 // Real: U^T forward (explicit diagonal) when asked, then L^T backward (kUnit, or
 // kDivide for an explicit diagonal, or kNone).
