@@ -1071,21 +1071,53 @@ struct SubstItem {
     double* x;
     int ldx, n, nrhs;
 };
-// A batch with many more columns than the GPU takes at once in the one-launch
-// solve (ctas: its CTAs of eight columns, each keeping a whole SM): there the
-// columns alone fill the GPU, and what counts is FP64 work per column. So the
-// triangles run one thread per column, and the updates, nearly all of the
-// work, on the tiled kernel, which shares each factor entry between 64
-// columns: 32-row blocks within blocks of kWideBlock rows, then the rows beyond
-// take kWideBlock steps in one launch (per 64 sweep matrices 12.5 ms of
-// updates at 128 steps a launch against 16.1 ms at 32; the one-launch solve
-// took 22 ms of the whole GPU).
+// The solve by blocks of many columns: the triangles run one thread per column,
+// and the updates, nearly all of the work, on the tiled kernel, which shares
+// each factor entry between 64 columns: 32-row blocks within blocks of
+// kWideBlock rows, then the rows beyond take kWideBlock steps in one launch (per
+// 64 sweep matrices 12.5 ms of updates at 128 steps a launch against 16.1 ms at
+// 32).
 constexpr int kWideBlock = 128;
-bool wide_batch(Context& ctx, const std::vector<SubstItem>& items) {
-    long long ctas = 0;
-    for (auto& it : items)
-        if (it.n > 2 * kWideBlock) ctas += (it.nrhs + 7) / 8;
-    return ctas >= 2 * ctx.num_sms;
+
+// Microseconds of both triangles, fitted to solves of 8 .. 12,000 (complex: ..
+// 8192) rows and up to 20,000 columns; the form that these favour was the
+// faster of the two, or within 5% of it (n <= 16: 18%, of 0.15 ms), at all 454
+// points. In one launch: a wave of a CTA per SM costs the latency of its row
+// blocks and the factor's way through every SM's L2 port, the more columns a
+// CTA has the less often.
+double one_launch_us(const Context& ctx, bool cplx, int n, long long nrhs) {
+    const int c = subst_cols_per_cta(ctx, cplx, n, nrhs);
+    const long long ctas = (nrhs + c - 1) / c, waves = (ctas + ctx.num_sms - 1) / ctx.num_sms;
+    const double block = c < 4 ? (cplx ? 0.2 : 0.1) : cplx ? (c == 8 ? 0.25 : 0.2) : c == 8 ? 0.2 : 0.15;
+    const double entry = cplx ? (c == 8 ? 0.7e-3 : c == 4 ? 0.41e-3 : c == 2 ? 0.33e-3 : 0.22e-3)
+                              : (c == 8 ? 0.24e-3 : c == 4 ? 0.18e-3 : c == 2 ? 0.105e-3 : 0.096e-3);
+    return (double)waves * ((cplx ? 10.0 : 5.0) + block * n + entry * n * n);
+}
+// By blocks: launches per row block, then FP64 work.
+double by_blocks_us(bool cplx, int n, long long nrhs) {
+    return cplx ? 3.7 * n + (double)nrhs * n * (1e-4 + 5.2e-7 * n) : 2.4 * n + (double)nrhs * n * (6e-5 + 2.6e-7 * n);
+}
+
+// Whether a solve goes by blocks: where the one launch takes longer (real n =
+// 12,000, 592 columns: 85 ms against 78, 296: 53, 65; complex n = 8192, 440: 77,
+// 68; real n = 2048, 2500: 5.7, 9.8; n = 16, 20,000: 0.29, 0.20). Beside other
+// batch workers' launches the blocks' latencies are filled, and what counts is
+// the GPU's time: the one-launch solve, whose CTAs keep a whole SM each, took
+// 22 ms of it per 64 sweep matrices. There batches of two CTAs of eight columns
+// per SM go by blocks (orders above two blocks).
+bool by_blocks(const Context& ctx, bool cplx, const std::vector<SubstItem>& items) {
+    if (ctx.concurrent) {
+        long long ctas = 0;
+        for (auto& it : items)
+            if (it.n > 2 * kWideBlock) ctas += (it.nrhs + 7) / 8;
+        return ctas >= 2 * ctx.num_sms;
+    }
+    double one = 0.0, blocks = 0.0;
+    for (auto& it : items) {
+        one += one_launch_us(ctx, cplx, it.n, it.nrhs);
+        blocks += by_blocks_us(cplx, it.n, it.nrhs);
+    }
+    return one > blocks;
 }
 
 void substitute_wide(Context& ctx, bool cplx, bool upper, bool lower_divides, const std::vector<SubstItem>& items) {
@@ -1119,7 +1151,7 @@ void substitute_wide(Context& ctx, bool cplx, bool upper, bool lower_divides, co
 }
 
 void substitute(Context& ctx, bool cplx, bool upper, bool lower_divides, const std::vector<SubstItem>& all) {
-    if (wide_batch(ctx, all)) {
+    if (by_blocks(ctx, cplx, all)) {
         substitute_wide(ctx, cplx, upper, lower_divides, all);
         return;
     }
@@ -1589,7 +1621,7 @@ void getrs_batch(Context& ctx, std::vector<SolveItem>& items, bool adjoint) {
         std::vector<SubstItem> all;
         for (auto& it : items)
             all.push_back(SubstItem{it.lu->p, it.lu->ld(), it.b->p, it.b->ld(), it.lu->rows, it.nrhs});
-        const bool wide = wide_batch(ctx, all);
+        const bool wide = by_blocks(ctx, cplx, all);
         std::vector<SubstItem> subst;  // the items solved by blocks
         for (size_t q = 0; q < items.size(); ++q) {
             auto& it = items[q];

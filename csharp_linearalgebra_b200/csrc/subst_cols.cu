@@ -514,6 +514,17 @@ void launch(Context& ctx, std::vector<ColsDesc>& v, int nmax, LowerKind lower, b
     ctx.kernel_launches++;
 }
 
+// The most columns per CTA (each reads the factors once) that still give four
+// SMs in five a CTA and fit shared memory; ctas(c): the CTAs of c columns.
+template <bool CPLX, class F>
+int columns_per_cta(const Context& ctx, int nmax, F&& ctas) {
+    const long long want = ctx.num_sms * 4 / 5;
+    if (ctas(8) >= want && Layout<CPLX, 8>::bytes(nmax) <= kMaxSmem) return 8;
+    if (ctas(4) >= want && Layout<CPLX, 4>::bytes(nmax) <= kMaxSmem) return 4;
+    if (ctas(2) >= want && Layout<CPLX, 2>::bytes(nmax) <= kMaxSmem) return 2;
+    return 1;
+}
+
 template <bool CPLX>
 void run(Context& ctx, LowerKind lower, bool upper, const std::vector<SubstCols>& items) {
     std::vector<ColsDesc> v;
@@ -531,12 +542,10 @@ void run(Context& ctx, LowerKind lower, bool upper, const std::vector<SubstCols>
         for (auto& d : v) t += (d.s.nrhs + c - 1) / c;
         return t;
     };
-    // The most columns per CTA (each reads the factors once) that still give
-    // four SMs in five a CTA and fit shared memory.
-    const long long want = ctx.num_sms * 4 / 5;
-    if (ctas(8) >= want && Layout<CPLX, 8>::bytes(nmax) <= kMaxSmem) launch<CPLX, 8>(ctx, v, nmax, lower, upper);
-    else if (ctas(4) >= want && Layout<CPLX, 4>::bytes(nmax) <= kMaxSmem) launch<CPLX, 4>(ctx, v, nmax, lower, upper);
-    else if (ctas(2) >= want && Layout<CPLX, 2>::bytes(nmax) <= kMaxSmem) launch<CPLX, 2>(ctx, v, nmax, lower, upper);
+    const int c = columns_per_cta<CPLX>(ctx, nmax, ctas);
+    if (c == 8) launch<CPLX, 8>(ctx, v, nmax, lower, upper);
+    else if (c == 4) launch<CPLX, 4>(ctx, v, nmax, lower, upper);
+    else if (c == 2) launch<CPLX, 2>(ctx, v, nmax, lower, upper);
     else launch<CPLX, 1>(ctx, v, nmax, lower, upper);
 }
 
@@ -545,6 +554,11 @@ void run(Context& ctx, LowerKind lower, bool upper, const std::vector<SubstCols>
 int subst_cols_max_order(bool cplx) {
     const size_t fixed = cplx ? Layout<true, 1>::bytes(0) : Layout<false, 1>::bytes(0);
     return (int)((kMaxSmem - fixed) / (cplx ? 16 : 8));
+}
+
+int subst_cols_per_cta(const Context& ctx, bool cplx, int n, long long nrhs) {
+    auto ctas = [&](int c) { return (nrhs + c - 1) / c; };
+    return cplx ? columns_per_cta<true>(ctx, n, ctas) : columns_per_cta<false>(ctx, n, ctas);
 }
 
 void subst_cols(Context& ctx, bool cplx, LowerKind lower, bool upper, const std::vector<SubstCols>& items) {

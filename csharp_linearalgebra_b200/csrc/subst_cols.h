@@ -22,6 +22,8 @@ struct SubstCols {
 
 // Largest order: one right-hand side's column fits a CTA's shared memory.
 int subst_cols_max_order(bool cplx);
+// Right-hand sides that a CTA takes (8, 4, 2 or 1) of one item of that order.
+int subst_cols_per_cta(const Context& ctx, bool cplx, int n, long long nrhs);
 // The lower solve (unit, or with an explicit diagonal, or none) and then the
 // upper solve (when asked) of every item, in one launch.
 void subst_cols(Context& ctx, bool cplx, LowerKind lower, bool upper, const std::vector<SubstCols>& items);
