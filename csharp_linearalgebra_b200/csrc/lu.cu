@@ -1120,7 +1120,7 @@ bool by_blocks(const Context& ctx, bool cplx, const std::vector<SubstItem>& item
     return one > blocks;
 }
 
-void substitute_wide(Context& ctx, bool cplx, bool upper, bool lower_divides, const std::vector<SubstItem>& items) {
+void substitute_blocks(Context& ctx, bool cplx, bool upper, bool lower_divides, const std::vector<SubstItem>& items) {
     constexpr int B = kWideBlock, D = kSubstBlock;
     int steps = 0;
     for (auto& it : items) steps = std::max(steps, (it.n + B - 1) / B);
@@ -1151,39 +1151,19 @@ void substitute_wide(Context& ctx, bool cplx, bool upper, bool lower_divides, co
 }
 
 void substitute(Context& ctx, bool cplx, bool upper, bool lower_divides, const std::vector<SubstItem>& all) {
-    if (by_blocks(ctx, cplx, all)) {
-        substitute_wide(ctx, cplx, upper, lower_divides, all);
-        return;
-    }
-    // Orders whose columns fit shared memory: one launch (subst_cols.cu).
+    const bool blocks = by_blocks(ctx, cplx, all);
+    // One launch (subst_cols.cu) where that is the faster form and the columns
+    // fit shared memory.
     std::vector<SubstCols> cols;
-    std::vector<SubstItem> items;
+    std::vector<SubstItem> rest;
     for (auto& it : all) {
-        if (it.n <= subst_cols_max_order(cplx)) cols.push_back(SubstCols{it.f, it.ldf, it.x, it.ldx, it.n, it.nrhs, nullptr});
-        else items.push_back(it);
+        if (!blocks && it.n <= subst_cols_max_order(cplx))
+            cols.push_back(SubstCols{it.f, it.ldf, it.x, it.ldx, it.n, it.nrhs, nullptr});
+        else
+            rest.push_back(it);
     }
     subst_cols(ctx, cplx, upper ? LowerKind::kNone : lower_divides ? LowerKind::kDivide : LowerKind::kUnit, upper, cols);
-    constexpr int B = kSubstBlock;
-    int steps = 0;
-    for (auto& it : items)
-        if (it.n > 0 && it.nrhs > 0) steps = std::max(steps, (it.n + B - 1) / B);
-    for (int s = 0; s < steps; ++s) {
-        std::vector<SubstDiagDesc> diag;
-        std::vector<SubstUpdateDesc> upd;
-        for (auto& it : items) {
-            const int n = it.n;
-            if (n == 0 || it.nrhs == 0) continue;
-            const int blocks = (n + B - 1) / B;
-            if (s >= blocks) continue;
-            const int k0 = (upper ? blocks - 1 - s : s) * B, w = std::min(B, n - k0);
-            diag.push_back(SubstDiagDesc{it.f, it.ldf, it.x, it.ldx, it.nrhs, k0, w});
-            const int r0 = upper ? 0 : k0 + w, r1 = upper ? k0 : n;
-            if (r1 > r0)
-                upd.push_back(SubstUpdateDesc{it.f, it.ldf, it.x, it.ldx, it.nrhs, r0, r1, k0, k0 + w,
-                                              (r1 - r0 + 63) / 64, 0});
-        }
-        launch_subst_step(ctx, cplx, upper, diag, upd, lower_divides);
-    }
+    substitute_blocks(ctx, cplx, upper, lower_divides, rest);
 }
 
 // ---------------------------------------------------------------------------

@@ -57,3 +57,15 @@ def test_large_orders_go_by_blocks(ws):
         return min(times)
 
     assert least(1776) < 1.9 * least(592)
+
+
+def test_order_beyond_one_launch(ws, orc):
+    """A complex order whose columns do not fit a CTA's shared memory (9664)."""
+    n = 9700
+    rng = np.random.default_rng(2)
+    u, v = rng.uniform(-1, 1, n) + 1j * rng.uniform(-1, 1, n), rng.uniform(-1, 1, n) / n
+    a = np.multiply.outer(v, u).T  # column-major
+    a[np.arange(n), np.arange(n)] += 2.0
+    b = rng.uniform(-1, 1, (n, 2)) + 1j * rng.uniform(-1, 1, (n, 2))
+    for tri in ("upper", "lower_unit"):
+        assert np.array_equal(ws.solve_triangular(tri, a, b), orc.trsolve(tri, a, b)), tri
