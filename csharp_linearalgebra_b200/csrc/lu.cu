@@ -1733,11 +1733,21 @@ void getrs(Context& ctx, const DMat& lu, const int* d_piv, DMat& b, int nrhs, bo
     getrs_batch(ctx, items, adjoint);
 }
 
-// The precision form's solves of up to this many columns take the one-launch
-// solve (2.1 ms for 64 columns of 4096 rows, 4.2 by blocks and updates). A
-// whole solve, n = 4096: 53.97 ms by blocks and 43.93 in one launch with 64
-// columns, 61.8 and 57.5 with 512, 72.3 and 79.1 with 1024.
-constexpr int kOneLaunchCols = 512;
+namespace {
+// The precision form's solves take the one launch where it ends before the
+// blocked triangular solves with DMMA updates, whose microseconds for both
+// triangles are fitted to whole solves of 300 .. 12,000 rows (complex: .. 6000)
+// and up to 2048 columns (n = 4096: 64 columns 24.3 ms by blocks and 20.0 in one
+// launch, 512 28.3 and 25.5, 1024 33.4 and 35.4; n = 8192, 512: 75.8, 83.9; n =
+// 12,000, 64: 112, 118, 512: 142, 223; complex n = 1024, 2048: 16.1, 13.6; n =
+// 6000, 512: 108, 133).
+bool free_order_ends_first(const Context& ctx, bool cplx, int n, long long cols) {
+    if (n > subst_cols_max_order(cplx)) return true;
+    const double whole = round_up(n, 64), entries = (double)cols * n * n;
+    const double free_us = cplx ? 2.0 * whole + 5.3e-7 * entries : whole + 1.05e-7 * entries;
+    return free_us < one_launch_us(ctx, cplx, n, cols);
+}
+}  // namespace
 
 void getrs_free_order(Context& ctx, const DMat& lu, const int* d_piv, DMat& b, int nrhs, bool adjoint) {
     const int n = lu.rows;
@@ -2034,8 +2044,8 @@ void gesv_mixed_pivoted(Context& ctx, const DMat& a, const DMat& b, DMat& x, int
     // The precision form's solves have no reference order to keep: blocked
     // triangular solves with DMMA updates.
     auto lu_solve = [&](DMat& m) {
-        if (nrhs <= kOneLaunchCols) getrs(ctx, f, piv.as<int>(), m, nrhs, false);
-        else getrs_free_order(ctx, f, piv.as<int>(), m, nrhs, false);
+        if (free_order_ends_first(ctx, f.cplx, f.rows, nrhs)) getrs_free_order(ctx, f, piv.as<int>(), m, nrhs, false);
+        else getrs(ctx, f, piv.as<int>(), m, nrhs, false);
     };
     lu_solve(x);
     const double ainf = norminf(ctx, a);
@@ -2720,14 +2730,14 @@ bool gesv_mixed_butterfly(Context& ctx, const DMat& a, const DMat& b, DMat& x, i
     };
     // (LU)^-1 or (LU)^-H in place: a few columns (the estimator's probes)
     // through the chained solve, more through the one-launch solve (its
-    // interchanges the identity), many by blocked TRSM + DMMA updates.
+    // interchanges the identity), or by blocked TRSM + DMMA updates.
     DBuf identity(ctx, sizeof(int) * (size_t)N);
     std::vector<int> order(N);
     for (int i = 0; i < N; ++i) order[i] = i;
     TNS_CUDA(cudaMemcpyAsync(identity.p, order.data(), sizeof(int) * N, cudaMemcpyHostToDevice, ctx.stream));
     auto lu_solve = [&](DMat& m, int cols, bool adjoint) {
         if (cols <= 2 * kChainCols) chain_solve(ctx, f, inverses.as<double>(), m, cols, adjoint);
-        else if (cols <= kOneLaunchCols && !adjoint) getrs(ctx, f, identity.as<int>(), m, cols, false);
+        else if (!adjoint && !free_order_ends_first(ctx, f.cplx, N, cols)) getrs(ctx, f, identity.as<int>(), m, cols, false);
         else getrs_free_order(ctx, f, nullptr, m, cols, adjoint);
     };
     // M := A^-1 M or A^-H M in place on an N-row panel (zeros below row n).
