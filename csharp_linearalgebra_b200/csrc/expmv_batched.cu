@@ -790,8 +790,6 @@ int resident_ctas(Context& ctx) {
     return per_sm * ctx.num_sms;
 }
 
-// One kernel instance per (element type, layout, skip form); L null: only the
-// count of resident CTAs.
 // What the host needs of a launch's Shape.
 struct Layout {
     int cols, unit, rows, lanes;  // panel pitch, rows per step, rows per box at most, resident CTAs

@@ -17,10 +17,11 @@
 // the reference bit for bit. In a batch, step k of every matrix runs in one
 // launch per phase (a grouped GEMM for the trailing updates).
 //
-// Solves: forward and backward substitution in the reference's order, blocked
-// into diagonal solves and register-tiled updates (one launch for a single
-// system, subst_cols.cu) that continue each element's chain of roundings in the reference's order, so A^-1 B -- the Pade
-// solve included -- matches the reference bit for bit. The adjoint solves,
+// Solves: forward and backward substitution in the reference's order, in one
+// launch (subst_cols.cu) or blocked into diagonal solves and register-tiled
+// updates, each of which continues every element's chain of roundings in that
+// order, so A^-1 B -- the Pade solve included -- matches the reference bit for
+// bit. The adjoint solves,
 // whose reference order is an inner product per row, run left-looking: ColumnOps.Dot's
 // vector order for real factors, sequential sums for complex ones (the forward
 // half of the complex adjoint, whose sums run in ascending k, right-looking
@@ -588,8 +589,8 @@ __global__ void trsm_kernel(const __grid_constant__ Batch<TrsmDesc> bt) {
 // kernels skip only when all four x[k] are zero, which can change nothing but
 // the sign of a zero). So each x[i] receives one chain of roundings in the
 // order of k, and the chains of different (row, column) pairs are
-// independent. The rows are cut into blocks of 32; for each block, in the
-// order of k:
+// independent. Where one launch is the slower form (by_blocks), the rows are cut
+// into blocks; for each block, in the order of k:
 //   1. solve_diag_blocks (subst_cols.cu) solves the block's own triangle,
 //      which completes x[k] for every k of the block;
 //   2. subst_update_kernel applies the block's steps to every row beyond it,
@@ -598,8 +599,8 @@ __global__ void trsm_kernel(const __grid_constant__ Batch<TrsmDesc> bt) {
 // the reference's operations in the reference's order and the solution
 // matches bit for bit; step 2, all but about 32/n of the work, runs as a
 // register-tiled product on every SM. The adjoint solves accumulate row by
-// row in the reference (dot products), an order a right-looking sweep cannot
-// reproduce; they stay on the blocked GEMM path.
+// row in the reference (dot products), an order that a right-looking sweep
+// cannot reproduce; they run left-looking, below.
 constexpr int kSubstBlock = kDiagBlock;
 
 struct SubstUpdateDesc {
@@ -884,7 +885,7 @@ __global__ void gather_rows_kernel(const __grid_constant__ Batch<GatherDesc> b) 
     }
 }
 constexpr int kGatherMaxCols = 128;
-constexpr int kGatherMaxRows = 24576;  // perm + pivots in 192 KB of shared memory
+constexpr int kGatherMaxRows = 24576;  // build_perm_kernel's last and root in 192 KB of shared memory
 
 // One tall panel over all SMs (panel_coop_kernel), when every CTA's slab fits
 // shared memory.

@@ -22,15 +22,8 @@
 //             reach the rows of block p + 1 (that 32 x 32 piece of the factor
 //             staged in shared memory), then step k of the triangle broadcasts
 //             x[k] by shuffles and every later lane continues its chain. The
-//             diagonal divisions use the correctly rounded reciprocal of the
-//             divisor, formed once per block, and two fused-multiply-add
-//             corrections, which end in the correctly rounded quotient (P. W.
-//             Markstein, "Computation of elementary functions on the IBM RISC
-//             System/6000 processor", IBM J. Res. Dev. 34 (1990): with
-//             y = RN(1/b), a q within one ulp of a/b and r = a - b q by a fused
-//             multiply-add, RN(q + r y) = RN(a/b)); operands outside
-//             [2^-500, 2^500] divide. A dependent division costs 113 cycles,
-//             this 40.
+//             diagonal divisions use the divisor's reciprocal, prepared once per
+//             block (divide.cuh): 40 cycles in the chain for a division's 113.
 //   update    a warp takes 32 rows (64 real) of all C columns, a row (two) and
 //             its C values per thread in registers, block p's solved x
 //             broadcast from shared memory, the factor's columns read from L2
