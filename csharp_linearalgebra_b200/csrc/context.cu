@@ -117,7 +117,7 @@ const void* Context::upload(const void* src, size_t bytes) {
             if (h_ring) {
                 old_rings.emplace_back(h_ring, d_ring);
                 h_ring = d_ring = nullptr;
-                ring_cap = 0;
+                ring_cap = ring_pos = hold_from = 0;  // no room anywhere, should the new one be refused
             }
             if (!ring_held) free_old_rings();
             char *host = nullptr, *dev = nullptr;
